@@ -888,6 +888,17 @@ __device__ __forceinline__ int fix_mul(float a, float b) {
     return __float_as_int(__fmaf_rn(a, b, 12582912.0f)) - 0x4B400000;
 }
 
+// The exponent k of the scale 2^k for a bound b on a node's sum: 29 - floor(log2 b) within +-120,
+// read from b's exponent field (a handful of integer instructions where ilogbf, ldexpf and the
+// scale's reciprocal by division took about sixty per thread); 0 for b = 0, -120 for a bound
+// that overflowed.
+__device__ __forceinline__ int fix_exponent(float b) {
+    const int e = __float_as_int(b) >> 23;
+    const int k = max(-120, min(120, 156 - e));
+    return b > 0.f ? (e == 255 ? -120 : k) : 0;
+}
+__device__ __forceinline__ float pow2(int k) { return __int_as_float((k + 127) << 23); }  // |k| <= 126
+
 struct Tile {
     int t[4][TWORDS];  // momentum x, y, z, mass
     float red[2][32];  // per-warp payload bounds
@@ -924,9 +935,10 @@ __device__ __forceinline__ void locate(const mpm_instance& I, const float* x, in
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const float xi = x[d] * I.inv_dx;
-        const float bf = floorf(xi - 0.5f);
-        base[d] = (int)fminf(fmaxf(bf, -1e8f), 1e8f) - I.lower_cell[d];
-        fx[d] = xi - bf;
+        // the conversion saturates, so an x far outside the grid stays outside it
+        const int b = __float2int_rd(xi - 0.5f);
+        base[d] = b - I.lower_cell[d];
+        fx[d] = xi - (float)b;
     }
 }
 
@@ -1299,8 +1311,8 @@ __device__ __forceinline__ void scatter_flush(Tile& T, const Payload& o, const m
     }
     const float nin = (float)max(cnt, 256);
     // scale = 2^(29 - floor(log2(n * B))): n * B * scale < 2^30
-    const float sq = Bq > 0.f ? ldexpf(1.f, max(-120, min(120, 29 - ilogbf(nin * Bq)))) : 1.f;
-    const float sm = Bm > 0.f ? ldexpf(1.f, max(-120, min(120, 29 - ilogbf(nin * Bm)))) : 1.f;
+    const int kq = fix_exponent(nin * Bq), km = fix_exponent(nin * Bm);
+    const float sq = pow2(kq), sm = pow2(km);
     uint32_t sw[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};  // CPIC: separated nodes
     if (o.live) {
         float wx[3], wy[3], wz[3];
@@ -1411,7 +1423,7 @@ __device__ __forceinline__ void scatter_flush(Tile& T, const Payload& o, const m
     }
     __syncthreads();
     // flush non-empty tile nodes, one 16-byte reduction each, zeroing the tile behind it
-    const float iq = 1.f / sq, im = 1.f / sm;
+    const float iq = pow2(-kq), im = pow2(-km);
 #pragma unroll
     for (int k = 0; k < TN / P; ++k) {
         const uint32_t d = nd[threadIdx.x + k * P];

@@ -33,6 +33,20 @@ constexpr int kSvdUnroll = GBM_SVD_UNROLL;
 #define GBM_SVD_TOL 1e-7f
 #endif
 
+// Approximate reciprocal square root and quotient, flushing subnormals: the arguments below are
+// kept above 1e-37 (or the result is selected away), and the default forms spend three to four
+// instructions each on scaling subnormal inputs.
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float quot_ftz(float a, float b) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return a * r;
+}
+
 // One Jacobi rotation in plane (P, Q) of the symmetric matrix a, accumulated into v.
 template <int P, int Q>
 __device__ __forceinline__ void jacobi_pq(float (&a)[3][3], float (&v)[3][3]) {
@@ -49,10 +63,10 @@ __device__ __forceinline__ void jacobi_pq(float (&a)[3][3], float (&v)[3][3]) {
     const float d = aqq - app;
     const float e = 2.f * apq;
     const float r2 = fmaf(d, d, e * e);
-    const float den = fabsf(d) + r2 * rsqrtf(fmaxf(r2, 1e-37f));
-    float t = __fdividef(e, copysignf(den, d));
+    const float den = fabsf(d) + r2 * rsqrt_ftz(fmaxf(r2, 1e-37f));
+    float t = quot_ftz(e, copysignf(den, d));
     t = (fabsf(apq) > 1e-18f) ? t : 0.f;
-    const float c = rsqrtf(1.f + t * t);
+    const float c = rsqrt_ftz(1.f + t * t);
     const float s = t * c;
     a[P][P] = app - t * apq;
     a[Q][Q] = aqq + t * apq;
@@ -87,10 +101,10 @@ __device__ __forceinline__ void onesided_pq(float (&b)[3][3], float (&v)[3][3]) 
     const float d = aqq - app;
     const float e = 2.f * apq;
     const float r2 = fmaf(d, d, e * e);
-    const float den = fabsf(d) + r2 * rsqrtf(fmaxf(r2, 1e-37f));
-    float t = __fdividef(e, copysignf(den, d));
+    const float den = fabsf(d) + r2 * rsqrt_ftz(fmaxf(r2, 1e-37f));
+    float t = quot_ftz(e, copysignf(den, d));
     t = (fabsf(apq) > 1e-30f) ? t : 0.f;
-    const float c = rsqrtf(1.f + t * t);
+    const float c = rsqrt_ftz(1.f + t * t);
     const float s = t * c;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -183,16 +197,26 @@ __device__ __forceinline__ void svd3(const float* A, float* U, float* S, float* 
             n2 = b[0][2] * b[0][2] + b[1][2] * b[1][2] + b[2][2] * b[2][2];
         }
     }
-    if (n0 < n1) swap_cols_neg<0, 1>(b, v, n0, n1);
-    if (n0 < n2) swap_cols_neg<0, 2>(b, v, n0, n2);
-    if (n1 < n2) swap_cols_neg<1, 2>(b, v, n1, n2);
+    // The decreasing order matters only where a column is small against another (the
+    // Gram-Schmidt below then takes the large ones first) or det A < 0 (the last singular value
+    // carries the sign): every use of U, S, V is symmetric in the order.  Decided per warp; the
+    // three conditional swaps are about fifty instructions.
+    const float nmax = fmaxf(n0, fmaxf(n1, n2)), nmin = fminf(n0, fminf(n1, n2));
+    const float det = b[0][0] * (b[1][1] * b[2][2] - b[2][1] * b[1][2]) +
+                      b[1][0] * (b[2][1] * b[0][2] - b[0][1] * b[2][2]) +
+                      b[2][0] * (b[0][1] * b[1][2] - b[1][1] * b[0][2]);
+    if (__any_sync(__activemask(), !(nmin > 0.0625f * nmax && det > 0.f))) {
+        if (n0 < n1) swap_cols_neg<0, 1>(b, v, n0, n1);
+        if (n0 < n2) swap_cols_neg<0, 2>(b, v, n0, n2);
+        if (n1 < n2) swap_cols_neg<1, 2>(b, v, n1, n2);
+    }
     // QR of B by Gram-Schmidt: u0 = b0 / |b0|, u1 = the part of b1 orthogonal to u0,
     // normalised, u2 = u0 x u1 (so det U = +1), R's diagonal (|b0|, |b1 - (u0.b1) u0|, u2.b2).
     // This is the QR with r00, r11 >= 0 (unique for rank >= 2).  A (near) zero b0 selects u0 = e_x; a b1 parallel to u0 selects for u1 the
     // unit vector orthogonal to u0 in the plane of u0 and the axis u0 is least aligned with.
     {
         const bool ok0 = n0 > 1e-30f;
-        const float r0 = rsqrtf(ok0 ? n0 : 1.f);
+        const float r0 = rsqrt_ftz(ok0 ? n0 : 1.f);
         const float u0[3] = {ok0 ? b[0][0] * r0 : 1.f, ok0 ? b[1][0] * r0 : 0.f, ok0 ? b[2][0] * r0 : 0.f};
         const float d01 = u0[0] * b[0][1] + u0[1] * b[1][1] + u0[2] * b[2][1];
         float w1[3] = {b[0][1] - d01 * u0[0], b[1][1] - d01 * u0[1], b[2][1] - d01 * u0[2]};
@@ -207,7 +231,7 @@ __device__ __forceinline__ void svd3(const float* A, float* U, float* S, float* 
             w1[2] = (k == 2 ? 1.f : 0.f) - uk * u0[2];
             m1 = w1[0] * w1[0] + w1[1] * w1[1] + w1[2] * w1[2];
         }
-        const float r1 = rsqrtf(m1);
+        const float r1 = rsqrt_ftz(m1);
         const float u1[3] = {w1[0] * r1, w1[1] * r1, w1[2] * r1};
         const float u2[3] = {u0[1] * u1[2] - u0[2] * u1[1], u0[2] * u1[0] - u0[0] * u1[2],
                              u0[0] * u1[1] - u0[1] * u1[0]};
