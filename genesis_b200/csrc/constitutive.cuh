@@ -84,9 +84,46 @@ __device__ __forceinline__ float flog(float x) { return GBM_FAST_MATH ? __logf(x
 __device__ __forceinline__ float fexp(float x) { return GBM_FAST_MATH ? __expf(x) : expf(x); }
 __device__ __forceinline__ float fdiv(float a, float b) { return GBM_FAST_MATH ? __fdividef(a, b) : a / b; }
 
-// Inviscid Liquid needs only J from the SVD (its stress is lam J (J - 1) I).
+// Elastic and Liquid need no more than J and, unless the model is neo-Hookean (elastic.py:78-81)
+// or the Liquid inviscid (its stress is lam J (J - 1) I), the polar rotation of F_tmp.
+__device__ __forceinline__ bool polar_suffices(const mpm_material& m) {
+    return m.kind == MPM_MAT_ELASTIC || m.kind == MPM_MAT_LIQUID;
+}
 __device__ __forceinline__ bool needs_uv(const mpm_material& m, float mu) {
+    if (m.kind == MPM_MAT_ELASTIC) return !(m.flags & MPM_MATF_NEOHOOKEAN);
     return !(m.kind == MPM_MAT_LIQUID && mu == 0.f);
+}
+
+// F_new and stress of Elastic and Liquid from J and R (R read only where needs_uv; Jp is kept)
+__device__ __forceinline__ void elastic_liquid(const mpm_material& m, float mu, float lam, float J, const float* Ft,
+                                               const float* R, float* F_new, float* stress) {
+    if (m.kind == MPM_MAT_LIQUID) {
+        // F_new = J^(1/3) I (liquid.py:52); pow(J, 1/3) is NaN for a negative J
+        const float c = J >= 0.f ? cbrtf(J) : __int_as_float(0x7fc00000);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) F_new[k] = (k % 4 == 0) ? c : 0.f;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) F_new[k] = Ft[k];
+    }
+    if (m.kind == MPM_MAT_ELASTIC && (m.flags & MPM_MATF_NEOHOOKEAN)) {
+        // mu F_tmp F_tmp^T + (lam log J - mu) I   (elastic.py:78-81)
+        const float d = lam * flog(J) - mu;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                float acc = Ft[i * 3 + 0] * Ft[j * 3 + 0] + Ft[i * 3 + 1] * Ft[j * 3 + 1] + Ft[i * 3 + 2] * Ft[j * 3 + 2];
+                stress[i * 3 + j] = mu * acc + (i == j ? d : 0.f);
+            }
+    } else if (m.kind == MPM_MAT_LIQUID && mu == 0.f) {
+        // liquid.py:47-48: mu is 0 unless viscous, so 2 mu (F_tmp - R) F_tmp^T vanishes
+        const float diag = lam * J * (J - 1.f);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) stress[k] = (k % 4 == 0) ? diag : 0.f;
+    } else {
+        corotated(mu, lam, J, Ft, R, stress);  // liquid.py:60 uses F_tmp
+    }
 }
 
 // Return mapping + stress for one particle.
@@ -96,43 +133,13 @@ __device__ __forceinline__ bool needs_uv(const mpm_material& m, float mu) {
 __device__ __forceinline__ void constitutive(const mpm_material& m, float mu, float lam, float eps, float J,
                                              const float* Ft, const float* U, const float* S, const float* V,
                                              float Jp, float* F_new, float& Jp_new, float* stress) {
-    float R[9];
     switch (m.kind) {
-        case MPM_MAT_ELASTIC: {
-#pragma unroll
-            for (int k = 0; k < 9; ++k) F_new[k] = Ft[k];
-            Jp_new = Jp;
-            if (m.flags & MPM_MATF_NEOHOOKEAN) {
-                // mu F_tmp F_tmp^T + (lam log J - mu) I   (elastic.py:78-81)
-                const float d = lam * flog(J) - mu;
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        float acc = Ft[i * 3 + 0] * Ft[j * 3 + 0] + Ft[i * 3 + 1] * Ft[j * 3 + 1] + Ft[i * 3 + 2] * Ft[j * 3 + 2];
-                        stress[i * 3 + j] = mu * acc + (i == j ? d : 0.f);
-                    }
-            } else {
-                uvt(U, V, R);
-                corotated(mu, lam, J, F_new, R, stress);
-            }
-            break;
-        }
+        case MPM_MAT_ELASTIC:
         case MPM_MAT_LIQUID: {
-            // F_new = J^(1/3) I (liquid.py:52); pow(J, 1/3) is NaN for a negative J
-            const float c = J >= 0.f ? cbrtf(J) : __int_as_float(0x7fc00000);
-#pragma unroll
-            for (int k = 0; k < 9; ++k) F_new[k] = (k % 4 == 0) ? c : 0.f;
+            float R[9];
+            uvt(U, V, R);
+            elastic_liquid(m, mu, lam, J, Ft, R, F_new, stress);
             Jp_new = Jp;
-            if (mu == 0.f) {
-                // liquid.py:47-48: mu is 0 unless viscous, so 2 mu (F_tmp - R) F_tmp^T vanishes
-                const float diag = lam * J * (J - 1.f);
-#pragma unroll
-                for (int k = 0; k < 9; ++k) stress[k] = (k % 4 == 0) ? diag : 0.f;
-            } else {
-                uvt(U, V, R);
-                corotated(mu, lam, J, Ft, R, stress);  // liquid.py:60 uses F_tmp
-            }
             break;
         }
         case MPM_MAT_ELASTOPLASTIC: {

@@ -1004,11 +1004,17 @@ __device__ __forceinline__ void particle_update(const mpm_instance& I, const mpm
 #pragma unroll
         for (int k = 0; k < 9; ++k) sv[(6 + k) * P] = C_in[k];
     }
-    float U[9], Sg[3], V[9];
-    svd3(Ft, U, Sg, V, needs_uv(m, mu));
-    const float J = Sg[0] * (Sg[1] * Sg[2]);
-    float Fn[9], stress[9], Jpn;
-    constitutive(m, mu, lam, I.eps, J, Ft, U, Sg, V, Jp, Fn, Jpn, stress);
+    float Fn[9], stress[9], Jpn, R[9], J;
+    // a warp of Elastic and Liquid particles takes J and R without the SVD
+    if (__all_sync(__activemask(), polar_suffices(m)) && polar3(Ft, needs_uv(m, mu), R, J)) {
+        elastic_liquid(m, mu, lam, J, Ft, R, Fn, stress);
+        Jpn = Jp;
+    } else {
+        float U[9], Sg[3], V[9];
+        svd3(Ft, U, Sg, V, needs_uv(m, mu));
+        J = Sg[0] * (Sg[1] * Sg[2]);
+        constitutive(m, mu, lam, I.eps, J, Ft, U, Sg, V, Jp, Fn, Jpn, stress);
+    }
     if (MUSCLE && (m.flags & MPM_MATF_MUSCLE) && par.actu) {
         // muscle.py:57-65: + stiffness * actu * F_tmp d d^T F_tmp^T; a Muscle is an Elastic,
         // whose F_new is F_tmp, so Fn stands in for F_tmp here

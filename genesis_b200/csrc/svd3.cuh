@@ -133,6 +133,59 @@ __device__ __forceinline__ void swap_cols_neg(float (&b)[3][3], float (&v)[3][3]
     nj = tn;
 }
 
+// cofactors K of A (K = det(A) A^-T)
+__device__ __forceinline__ void cofactor3(const float* A, float* K) {
+    K[0] = A[4] * A[8] - A[5] * A[7];
+    K[1] = A[5] * A[6] - A[3] * A[8];
+    K[2] = A[3] * A[7] - A[4] * A[6];
+    K[3] = A[2] * A[7] - A[1] * A[8];
+    K[4] = A[0] * A[8] - A[2] * A[6];
+    K[5] = A[1] * A[6] - A[0] * A[7];
+    K[6] = A[1] * A[5] - A[2] * A[4];
+    K[7] = A[2] * A[3] - A[0] * A[5];
+    K[8] = A[0] * A[4] - A[1] * A[3];
+}
+
+// J = det A and, where want_R, the rotation R of A's polar decomposition A = R S (= U V^T of its
+// SVD), by the Newton iteration X <- (X + X^-T) / 2 (Higham, SIAM J. Sci. Stat. Comput. 7, 1986):
+// quadratic, so the update that moves X by less than 2e-4 leaves an error below 2e-8.  Materials
+// that need no more than this (Elastic, Liquid) skip the SVD: two or three iterations of about
+// sixty instructions at the strains of a running scene, where the SVD takes about seven hundred.
+// The whole warp goes one way: returns false (nothing usable) where a lane has det A <= 0, is too
+// ill-conditioned for the determinant in float32 (|A|_F^6 >= 108 det^2: singular values (a, 1, 1)
+// pass for a in [0.3, 2.8]), or has not converged.
+__device__ __forceinline__ bool polar3(const float* A, bool want_R, float* R, float& J) {
+    const unsigned lanes = __activemask();
+    float K[9];
+    cofactor3(A, K);
+    J = A[0] * K[0] + A[1] * K[1] + A[2] * K[2];
+    float n2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        R[k] = A[k];
+        n2 = fmaf(A[k], A[k], n2);
+    }
+    if (!__all_sync(lanes, J > 1e-6f && n2 * n2 * n2 < 108.f * J * J)) return false;
+    if (!__any_sync(lanes, want_R)) return true;
+    float det = J;
+#pragma unroll 1
+    for (int it = 0; it < 8; ++it) {
+        const float h = quot_ftz(0.5f, det);
+        float mv = 0.f;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const float x = fmaf(h, K[k], 0.5f * R[k]);
+            const float d = x - R[k];
+            mv = fmaf(d, d, mv);
+            R[k] = x;
+        }
+        if (__all_sync(lanes, !want_R || mv < 4e-8f)) return true;
+        cofactor3(R, K);
+        det = R[0] * K[0] + R[1] * K[1] + R[2] * K[2];
+    }
+    return false;
+}
+
 // A (row-major, 9 floats) = U diag(S) V^T with U, V proper rotations (row-major).
 // need_uv = false: the caller uses only the product S0 S1 S2 (= det A, which the QR
 // below yields whatever V is), so this lane does not hold up the warp's Jacobi sweeps.
