@@ -175,10 +175,13 @@ __device__ __forceinline__ void constitutive(const mpm_material& m, float mu, fl
         }
         case MPM_MAT_SNOW: {
             float Sn[3];
+            float jp = Jp;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) Sn[d] = fminf(fmaxf(S[d], m.clamp_lo), m.clamp_hi);
-            // Jp prod(S / S_new) as one quotient (J is S0 (S1 S2): exactly 1 where nothing yields)
-            Jp_new = Jp * fdiv(J, Sn[0] * (Sn[1] * Sn[2]));
+            for (int d = 0; d < 3; ++d) {
+                Sn[d] = fminf(fmaxf(S[d], m.clamp_lo), m.clamp_hi);
+                jp = jp * fdiv(S[d], Sn[d]);
+            }
+            Jp_new = jp;
             usvt(U, Sn, V, F_new);
             // snow.py:75-79: hardening from the previous Jp
             const float h = fexp(10.f * (1.f - Jp));

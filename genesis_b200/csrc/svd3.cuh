@@ -189,8 +189,10 @@ __device__ __forceinline__ bool polar3(const float* A, bool want_R, float* R, fl
 // A (row-major, 9 floats) = U diag(S) V^T with U, V proper rotations (row-major).
 // need_uv = false: the caller uses only the product S0 S1 S2 (= det A, which the QR
 // below yields whatever V is), so this lane does not hold up the warp's Jacobi sweeps.
+// ordered = false: the caller takes U, S, V in any order where that changes no more than rounding.
 template <int SWEEPS = 4>
-__device__ __forceinline__ void svd3(const float* A, float* U, float* S, float* V, bool need_uv = true) {
+__device__ __forceinline__ void svd3(const float* A, float* U, float* S, float* V, bool need_uv = true,
+                                     bool ordered = true) {
     float a[3][3];
     // A^T A
 #pragma unroll
@@ -252,13 +254,13 @@ __device__ __forceinline__ void svd3(const float* A, float* U, float* S, float* 
     }
     // The decreasing order matters only where a column is small against another (the
     // Gram-Schmidt below then takes the large ones first) or det A < 0 (the last singular value
-    // carries the sign): every use of U, S, V is symmetric in the order.  Decided per warp; the
-    // three conditional swaps are about fifty instructions.
+    // carries the sign): the materials use U, S, V symmetrically.  Decided per warp; the three
+    // conditional swaps are about fifty instructions.
     const float nmax = fmaxf(n0, fmaxf(n1, n2)), nmin = fminf(n0, fminf(n1, n2));
     const float det = b[0][0] * (b[1][1] * b[2][2] - b[2][1] * b[1][2]) +
                       b[1][0] * (b[2][1] * b[0][2] - b[0][1] * b[2][2]) +
                       b[2][0] * (b[0][1] * b[1][2] - b[1][1] * b[0][2]);
-    if (__any_sync(__activemask(), !(nmin > 0.0625f * nmax && det > 0.f))) {
+    if (ordered || __any_sync(__activemask(), !(nmin > 0.0625f * nmax && det > 0.f))) {
         if (n0 < n1) swap_cols_neg<0, 1>(b, v, n0, n1);
         if (n0 < n2) swap_cols_neg<0, 2>(b, v, n0, n2);
         if (n1 < n2) swap_cols_neg<1, 2>(b, v, n1, n2);
