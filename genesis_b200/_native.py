@@ -43,6 +43,7 @@ PFLAG_ACTIVE = 1
 PFLAG_FREE = 2
 PROBF_NONFREE = 1
 PROBF_CPIC = 2
+PROBF_ROTATE = 4
 
 MAT_ELASTIC, MAT_ELASTOPLASTIC, MAT_LIQUID, MAT_SAND, MAT_SNOW = 0, 1, 2, 3, 4
 

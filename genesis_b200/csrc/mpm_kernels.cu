@@ -92,7 +92,8 @@ enum Counter {
     CNT_SORTED = 3,
     CNT_FALLBACK = 4 /* u64 at 4,5 */,
     CNT_DONE = 6,
-    CNT_GRID_OPS = 7  // grid ops run on this workspace (the NOISE force field's counter)
+    CNT_GRID_OPS = 7,  // grid ops run on this workspace (the NOISE force field's counter)
+    CNT_ROTATE = 8     // active-block counts of the two extra rotating grids
 };
 constexpr int N_COUNTERS = 16;
 
@@ -119,9 +120,18 @@ struct Ws {
     int64_t tmp_stride;
 };
 
+// One momentum grid with the list of blocks that hold anything.  Problems with
+// MPM_PROBF_ROTATE have three: one being read, one being accumulated, one being cleared.
+struct Grid {
+    float4* mm;
+    uint32_t* flag;
+    int2* active;
+    uint32_t* n_active;
+};
+
 static inline uint64_t align_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 
-constexpr int N_LAYOUT = 19;
+constexpr int N_LAYOUT = 25;
 
 struct Layout {
     uint64_t off[N_LAYOUT];
@@ -154,10 +164,18 @@ static Layout layout_of(const mpm_problem& p) {
         n * 4,                     // lam_tmp
         N_COUNTERS * 4,            // counters
         (uint64_t)p.n_instances * 4,  // per-instance status
+        0, 0, 0, 0, 0, 0,             // the two extra rotating grids: mm, flag, active
     };
+    if (p.flags & MPM_PROBF_ROTATE)
+        for (int k = 19; k < 25; k += 3) {
+            sizes[k] = nb * BLK3 * 16;
+            sizes[k + 1] = nb * 4;
+            sizes[k + 2] = nb * 8;
+        }
     uint64_t o = 0;
     for (int i = 0; i < N_LAYOUT; ++i) {
         L.off[i] = o;
+        if (i >= 19 && !sizes[i]) continue;
         o = align_up(o + (sizes[i] ? sizes[i] : 1), 256);
     }
     L.total = o;
@@ -189,6 +207,17 @@ static Ws ws_of(const mpm_problem& p, void* base) {
     w.inst_status = (uint32_t*)(b + L.off[18]);
     w.tmp_stride = (int64_t)align_up(p.n_particles > 0 ? p.n_particles : 1, 64);
     return w;
+}
+
+// grid k (0, 1, 2) of the rotation; 0 is the workspace's own
+static Grid grid_of(const mpm_problem& p, void* base, int k) {
+    const Ws w = ws_of(p, base);
+    if (k == 0) return Grid{w.mm, w.flag, w.active, &w.counters[CNT_ACTIVE]};
+    const Layout L = layout_of(p);
+    char* b = (char*)base;
+    const int o = 19 + 3 * (k - 1);
+    return Grid{(float4*)(b + L.off[o]), (uint32_t*)(b + L.off[o + 1]), (int2*)(b + L.off[o + 2]),
+                &w.counters[CNT_ROTATE + k - 1]};
 }
 
 // ---------------------------------------------------------------- helpers
@@ -271,17 +300,57 @@ __device__ __forceinline__ int64_t node_addr(const mpm_instance& I, int gx, int 
     return (I.blk_base + lb) * BLK3 + ln;
 }
 
-__device__ __forceinline__ void mark_block(Ws& w, int inst, const mpm_instance& I, int bx, int by, int bz) {
+__device__ __forceinline__ void mark_block(Ws& w, int inst, const mpm_instance& I, int bx, int by, int bz,
+                                           uint32_t* n_active) {
     const int lb = (bx * I.nblk[1] + by) * I.nblk[2] + bz;
     uint32_t* f = &w.flag[I.blk_base + lb];
     if (*((volatile uint32_t*)f) == 0u && atomicExch(f, 1u) == 0u) {
-        const int i = (int)atomicAdd(&w.counters[CNT_ACTIVE], 1u);
+        const int i = (int)atomicAdd(n_active, 1u);
         w.active[i] = make_int2(inst, pack_bc(bx, by, bz));
     }
 }
 
 __device__ __forceinline__ bool finite3(float a, float b, float c) {
     return isfinite(a) && isfinite(b) && isfinite(c);
+}
+
+// The grid op's MPM core (legacy_coupler.py:364-375, 495-496) on node (gx, gy, gz): velocity from
+// momentum and mass, gravity, then the boundary; zero where the mass is at most eps.
+__device__ __forceinline__ float4 node_velocity(const mpm_instance& I, const float4& mm, int gx, int gy, int gz) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (mm.w > I.eps) {
+        const float inv = 1.f / mm.w;  // (1 / mass) * vel_in (legacy_coupler.py:369)
+        v.x = inv * mm.x + I.dt * I.gravity[0];
+        v.y = inv * mm.y + I.dt * I.gravity[1];
+        v.z = inv * mm.z + I.dt * I.gravity[2];
+        v.x = bc_vel((float)(gx + I.lower_cell[0]) * I.dx, v.x, I.bnd_lo[0], I.bnd_hi[0]);
+        v.y = bc_vel((float)(gy + I.lower_cell[1]) * I.dx, v.y, I.bnd_lo[1], I.bnd_hi[1]);
+        v.z = bc_vel((float)(gz + I.lower_cell[2]) * I.dx, v.z, I.bnd_lo[2], I.bnd_hi[2]);
+    }
+    v.w = v.z;  // a copy of z for the packed gather
+    return v;
+}
+
+// Overlapped launches (programmatic stream serialization): the kernel's CTAs may become resident
+// while its predecessor still runs.  It calls pdl_wait() before it touches anything the predecessor
+// writes (the call returns once that has completed and its writes are visible), and pdl_trigger()
+// only after it.  So when a kernel's prologue runs, every kernel before its predecessor has
+// completed: the prologue may read what those wrote, never what the predecessor writes.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+static void launch_overlapped(void (*k)(P...), int grid, int block, cudaStream_t s, const A&... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, k, P(args)...);
 }
 
 // ---------------------------------------------------------------- sort
@@ -1272,7 +1341,7 @@ __device__ __forceinline__ void tile_zero(Tile& T, int P) {
 template <int P, bool CPIC = false>
 __device__ __forceinline__ void scatter_flush(Tile& T, const Payload& o, const mpm_instance& I, int inst,
                                               const BlockCoord& bc, int ox, int oy, int oz, Ws& w, const int* tab,
-                                              const uint32_t* nd, const P2GArgs* cp = nullptr) {
+                                              const uint32_t* nd, uint32_t* n_active, const P2GArgs* cp = nullptr) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float wbq = warp_max(o.in_tile ? o.bq : 0.f);
     const float wbm = warp_max(o.in_tile ? o.mass : 0.f);
@@ -1315,7 +1384,7 @@ __device__ __forceinline__ void scatter_flush(Tile& T, const Payload& o, const m
             if (e[a] == 0) on = on && ((rch >> (2 * a)) & 1u);
             if (e[a] == 2) on = on && ((rch >> (2 * a + 1)) & 1u);
         }
-        if (on) mark_block(w, inst, I, bc.bx + e[0] - 1, bc.by + e[1] - 1, bc.bz + e[2] - 1);
+        if (on) mark_block(w, inst, I, bc.bx + e[0] - 1, bc.by + e[1] - 1, bc.bz + e[2] - 1, n_active);
     }
     const float nin = (float)max(cnt, 256);
     // scale = 2^(29 - floor(log2(n * B))): n * B * scale < 2^30
@@ -1422,7 +1491,7 @@ __device__ __forceinline__ void scatter_flush(Tile& T, const Payload& o, const m
                         const float ay = o.q[1] + (o.A[3] * i + o.A[4] * j + o.A[5] * k);
                         const float az = o.q[2] + (o.A[6] * i + o.A[7] * j + o.A[8] * k);
                         atomicAdd(&w.mm[node_addr(I, gx, gy, gz)], make_float4(wt * ax, wt * ay, wt * az, wt * o.mass));
-                        mark_block(w, inst, I, gx >> 2, gy >> 2, gz >> 2);
+                        mark_block(w, inst, I, gx >> 2, gy >> 2, gz >> 2, n_active);
                     }
         }
     }
@@ -1483,7 +1552,8 @@ __device__ __forceinline__ void vel_tile_load(VelTile& VT, const Ws& w, const Nb
 // g2p gather (mpm_solver.py:396-431): v = sum w v_i, C = 4 inv_dx sum w v_i (off - fx)^T;
 // then x += dt v and the boundary (mpm_solver.py:434-437).  Returns false if nothing
 // could be gathered (non-finite x).
-template <int P, bool CPIC = false>
+// RAW: w.gv holds momentum and mass instead of velocities (k_g2p2g_rotate); VT holds velocities
+template <int P, bool CPIC = false, bool RAW = false>
 __device__ __forceinline__ bool gather(const VelTile& VT, const Ws& w, const mpm_instance& I, int inst, float* x,
                                        float* nv, float* nC, int ox, int oy, int oz, const P2GArgs* cp = nullptr,
                                        int p = 0) {
@@ -1615,7 +1685,8 @@ __device__ __forceinline__ bool gather(const VelTile& VT, const Ws& w, const mpm
                         set_status(w, inst, MPM_STATUS_OUT_OF_GRID);
                         continue;
                     }
-                    const float4 g = w.gv[node_addr(I, gx, gy, gz)];
+                    float4 g = w.gv[node_addr(I, gx, gy, gz)];
+                    if constexpr (RAW) g = node_velocity(I, g, gx, gy, gz);
                     const float wt = sel3(wx, i) * sel3(wy, j) * sel3(wz, k);
                     const float d0 = (float)i - fx[0], d1 = (float)j - fx[1], d2 = (float)k - fx[2];
                     nv[0] += wt * g.x;
@@ -1694,7 +1765,7 @@ __global__ void __launch_bounds__(P, kP2GCtasPerSM<P>) k_p2g(P2GArgs a) {
             }
             particle_update<P, MUSCLE>(I, a.mats, a.par, p, x, v, C, ox, oy, oz, o, w, ch.x, SH);
         }
-        scatter_flush<P, CPIC>(T, o, I, ch.x, bc, ox, oy, oz, w, nbt[tb], nd, &a);
+        scatter_flush<P, CPIC>(T, o, I, ch.x, bc, ox, oy, oz, w, nbt[tb], nd, &w.counters[CNT_ACTIVE], &a);
         tb ^= 1;
     }
 }
@@ -1805,8 +1876,108 @@ __global__ void __launch_bounds__(P, kP2GCtasPerSM<P>) k_g2p2g(P2GArgs a) {
                 particle_update<P, MUSCLE>(I, a.mats, a.par, p, x, nv, nC, ox, oy, oz, o, w, ch.x, SH);
             }
         }
-        scatter_flush<P, CPIC>(T, o, I, ch.x, bc, ox, oy, oz, w, nbt[tb], nd, &a);
+        scatter_flush<P, CPIC>(T, o, I, ch.x, bc, ox, oy, oz, w, nbt[tb], nd, &w.counters[CNT_ACTIVE], &a);
         tb ^= 1;
+    }
+}
+
+// g2p2g with the grid op folded in, for problems whose work items fit the GPU at once
+// (rotate_applies).  There a substep is one item's latency plus the grid op's, and two kernel
+// boundaries; here each item computes the velocities of its tile's nodes itself, from the
+// momentum that the kernel before accumulated (`in`), and accumulates into a grid (w) that the
+// kernel before that has cleared.  A node is updated by every item whose tile holds it (about
+// eight times), which idle SMs absorb: a full GPU does not (3.5% slower on the 500k scene).  The
+// CTAs clear the third grid, read two kernels ago, behind them.  The prologue runs beside the
+// kernel before.  us per substep against g2p2g + grid op (49 substeps, one B200): 1k elastic
+// particles 8.0 against 14.5, 32k 10.1 / 16.0, 16 environments of 2k muscle particles 11.4 / 17.5,
+// 80k snow 17.3 / 23.3, 125k sand 23.9 / 28.8, 216k elastic 31.3 / 36.7, 288k 41.1 / 43.9.
+constexpr int kRotateClearers = 148;
+template <int P, bool MUSCLE>
+__global__ void __launch_bounds__(P, kP2GCtasPerSM<P>) k_g2p2g_rotate(P2GArgs a, Grid old, uint32_t* n_out) {
+    __shared__ VelTile VT;
+    __shared__ Tile T;
+    __shared__ Stash<P> SH;
+    Ws& w = a.w;  // mm, flag, active (and n_out): the grid accumulated here; gv: the one read
+    const int n_chunks = (int)w.counters[CNT_CHUNKS];
+    // CTAs beyond the work items (and beyond one per SM, to clear the old grid) leave at once: left
+    // waiting they would hold the places of the next kernel's CTAs, which then pile up on a few SMs
+    // (32k particles: 14.0 us per substep with them, 9.9 without)
+    const int workers = min((int)gridDim.x, max(n_chunks, kRotateClearers));
+    if ((int)blockIdx.x >= workers) return;
+    const int64_t st = a.par.state_stride;
+    float* __restrict__ S = a.par.state;
+    __shared__ uint32_t nd[TN];
+#pragma unroll
+    for (int k = 0; k < TN / P; ++k) nd[threadIdx.x + k * P] = node_desc(threadIdx.x + k * P);
+    tile_zero(T, P);
+    int4 next = blockIdx.x < n_chunks ? w.chunks[blockIdx.x] : make_int4(0, 0, 0, 0);
+    __shared__ int nbt[2][27];
+    int tb = 0;
+    if ((int)blockIdx.x < n_chunks) nb_table(a.inst[next.x], unpack_bc(next.y), nbt[0]);
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    // clear the old grid, one block per 64 threads; the CTAs without a work item take the first
+    const int n_old = (int)*(volatile uint32_t*)old.n_active;
+    const int ln = threadIdx.x % BLK3;
+    for (int i = (workers - 1 - (int)blockIdx.x) * (P / BLK3) + (int)threadIdx.x / BLK3; i < n_old;
+         i += workers * (P / BLK3)) {
+        const int2 e = old.active[i];
+        const mpm_instance& I = a.inst[e.x];
+        const BlockCoord bc = unpack_bc(e.y);
+        const int64_t blk = I.blk_base + local_block(I, bc.bx, bc.by, bc.bz);
+        old.mm[blk * BLK3 + ln] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ln == 0) old.flag[blk] = 0u;
+    }
+    for (int ci = blockIdx.x; ci < n_chunks; ci += gridDim.x) {
+        const int4 ch = next;
+        if (ci + (int)gridDim.x < n_chunks) next = w.chunks[ci + gridDim.x];
+        const int p = ch.z + threadIdx.x;
+        const bool have = p < ch.w;
+        float x[3] = {0.f, 0.f, 0.f};
+        uint8_t pf = 0;
+        if (have) {
+            pf = a.par.pflags[p];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) x[d] = S[(MPM_CH_X + d) * st + p];
+        }
+        const mpm_instance& I = a.inst[ch.x];
+        const BlockCoord bc = unpack_bc(ch.y);
+        const int ox = bc.bx * BLK - MARGIN, oy = bc.by * BLK - MARGIN, oz = bc.bz * BLK - MARGIN;
+        float4 mm[TN / P];
+#pragma unroll
+        for (int k = 0; k < TN / P; ++k) {
+            const int64_t at = tab_addr(nbt[tb], nd[threadIdx.x + k * P]);
+            mm[k] = at >= 0 ? w.gv[at] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < TN / P; ++k) {
+            const uint32_t d = nd[threadIdx.x + k * P];
+            VT.v[(d >> 12) & 1023] = node_velocity(I, mm[k], ox + (int)((d >> 22) & 7), oy + (int)((d >> 25) & 7),
+                                                   oz + (int)((d >> 28) & 7));
+        }
+        __syncthreads();
+        if (ci + (int)gridDim.x < n_chunks) nb_table(a.inst[next.x], unpack_bc(next.y), nbt[tb ^ 1]);
+        Payload o;
+        o.live = o.in_tile = false;
+        o.mass = o.bq = 0.f;
+        if (have && (pf & MPM_PFLAG_ACTIVE)) {
+            float nv[3], nC[9];
+            if (gather<P, false, true>(VT, w, I, ch.x, x, nv, nC, ox, oy, oz)) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) S[(MPM_CH_X + d) * st + p] = x[d];
+                particle_update<P, MUSCLE>(I, a.mats, a.par, p, x, nv, nC, ox, oy, oz, o, w, ch.x, SH);
+            }
+        }
+        scatter_flush<P>(T, o, I, ch.x, bc, ox, oy, oz, w, nbt[tb], nd, n_out);
+        tb ^= 1;
+    }
+    // the last worker to finish empties the cleared grid's list (every one has read its length)
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&w.counters[CNT_DONE], 1u) == (uint32_t)workers - 1u) {
+        *old.n_active = 0u;
+        w.counters[CNT_DONE] = 0u;
+        w.counters[CNT_GRID_OPS] += 1u;
     }
 }
 
@@ -2010,8 +2181,8 @@ __global__ void __launch_bounds__(256, 4) k_grid_op(mpm_problem prob, const mpm_
                                                  const mpm_collider* __restrict__ colliders, int n_colliders,
                                                  float* collider_force, const float* __restrict__ sdf_voxels,
                                                  const mpm_force_field* __restrict__ ffs, int n_ff,
-                                                 const int* __restrict__ ff_perm, int count_op) {
-    const int n_active = (int)w.counters[CNT_ACTIVE];
+                                                 const int* __restrict__ ff_perm, int count_op, uint32_t* count, Grid old) {
+    const int n_active = (int)*count;
     const uint32_t ops = w.counters[CNT_GRID_OPS];
     const int gpc = blockDim.x / BLK3;
     const int grp = threadIdx.x / BLK3;
@@ -2069,13 +2240,24 @@ __global__ void __launch_bounds__(256, 4) k_grid_op(mpm_problem prob, const mpm_
         w.mm[g] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (ln == 0) w.flag[I.blk_base + lb] = 0u;
     }
+    if (old.mm) {  // the end of a rotating run: the grid read by its last k_g2p2g_rotate
+        const int n_old = (int)*old.n_active;
+        for (int i = blockIdx.x * gpc + grp; i < n_old; i += gridDim.x * gpc) {
+            const int2 e = old.active[i];
+            const BlockCoord bc = unpack_bc(e.y);
+            const int64_t blk = inst[e.x].blk_base + local_block(inst[e.x], bc.bx, bc.by, bc.bz);
+            old.mm[blk * BLK3 + ln] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ln == 0) old.flag[blk] = 0u;
+        }
+    }
     // the last CTA to finish resets the active-block count for the next p2g: every CTA read
     // the count into registers before this barrier, so no fence is needed; no CTA waits on
     // another
     __syncthreads();
     if (threadIdx.x == 0) {
         if (atomicAdd(&w.counters[CNT_DONE], 1u) == gridDim.x - 1) {
-            w.counters[CNT_ACTIVE] = 0u;
+            *count = 0u;
+            if (old.mm) *old.n_active = 0u;
             w.counters[CNT_DONE] = 0u;
             if (count_op) w.counters[CNT_GRID_OPS] = ops + 1u;
         }
@@ -2327,8 +2509,9 @@ static int launch_p2g(const mpm_problem* prob, const mpm_tables* tab, mpm_partic
 }
 
 // advance = false (the adjoint's recompute): the colliders keep their pose and accumulate no force
+// cur, old: the grids that a rotating run ends with (the one to update, the one to clear)
 static int launch_grid_op(const mpm_problem* prob, const mpm_tables* tab, void* ws, cudaStream_t s,
-                          bool advance = true) {
+                          bool advance = true, const Grid* cur = nullptr, const Grid* old = nullptr) {
     const DevInfo* d = dev_info();
     if (!d) return MPM_E_CUDA;
     int ctas = prob->grid_ctas > 0 ? prob->grid_ctas : d->sms * d->occ_grid;
@@ -2338,14 +2521,23 @@ static int launch_grid_op(const mpm_problem* prob, const mpm_tables* tab, void* 
     const int nc = tab->colliders ? tab->n_colliders : 0;
     if (tab->n_force_fields < 0 || (tab->n_force_fields > 0 && !tab->force_fields)) return MPM_E_INVALID;
     const int nff = tab->force_fields ? tab->n_force_fields : 0;
+    Ws w = ws_of(*prob, ws);
+    uint32_t* count = &w.counters[CNT_ACTIVE];
+    if (cur) {
+        w.mm = cur->mm;
+        w.flag = cur->flag;
+        w.active = cur->active;
+        count = cur->n_active;
+    }
+    const Grid none{nullptr, nullptr, nullptr, nullptr};
     if (nff > 0)
-        k_grid_op<true><<<ctas, 256, 0, s>>>(*prob, tab->instances, ws_of(*prob, ws), tab->colliders, nc,
+        k_grid_op<true><<<ctas, 256, 0, s>>>(*prob, tab->instances, w, tab->colliders, nc,
                                               advance ? tab->collider_force : nullptr, tab->sdf_voxels,
-                                              tab->force_fields, nff, tab->ff_perm, advance ? 1 : 0);
+                                              tab->force_fields, nff, tab->ff_perm, advance ? 1 : 0, count, none);
     else
-        k_grid_op<false><<<ctas, 256, 0, s>>>(*prob, tab->instances, ws_of(*prob, ws), tab->colliders, nc,
+        k_grid_op<false><<<ctas, 256, 0, s>>>(*prob, tab->instances, w, tab->colliders, nc,
                                                advance ? tab->collider_force : nullptr, tab->sdf_voxels, nullptr, 0,
-                                               nullptr, advance ? 1 : 0);
+                                               nullptr, advance ? 1 : 0, count, old ? *old : none);
     if (nc > 0 && advance)
         k_advance_colliders<<<(nc + 63) / 64, 64, 0, s>>>(tab->instances, prob->n_instances, tab->colliders, nc);
     return cuda_ok();
@@ -2365,6 +2557,36 @@ static int launch_g2p(const mpm_problem* prob, const mpm_tables* tab, mpm_partic
         case 256: run_g2p<256>(cpic, ctas, s, a); break;
         case 512: run_g2p<512>(cpic, ctas, s, a); break;
     }
+    return cuda_ok();
+}
+
+// Whether a run uses k_g2p2g_rotate: the workspace has the extra grids, work items of 128
+// particles, and nothing acts on the grid but gravity and the boundary (a collider's reaction
+// would be counted once per tile; non-free particles and CPIC work on the grid between the
+// kernels).
+static bool rotate_applies(const mpm_problem* prob, const mpm_tables* tab) {
+    return (prob->flags & MPM_PROBF_ROTATE) && !(prob->flags & (MPM_PROBF_NONFREE | MPM_PROBF_CPIC)) &&
+           prob->chunk_particles == 128 && !(tab->colliders && tab->n_colliders > 0) &&
+           !(tab->force_fields && tab->n_force_fields > 0);
+}
+
+// substep i (counted from the run's p2g) reads grid i - 1, accumulates grid i, clears grid i + 1 (mod 3)
+static int launch_rotate(const mpm_problem* prob, const mpm_tables* tab, mpm_particles* par, void* ws, int32_t i,
+                         cudaStream_t s) {
+    const DevInfo* d = dev_info();
+    if (!d) return MPM_E_CUDA;
+    P2GArgs a;
+    bool cpic;
+    int rc = p2g_args(prob, tab, par, ws, a, cpic);
+    if (rc) return rc;
+    const Grid in = grid_of(*prob, ws, (i - 1) % 3), out = grid_of(*prob, ws, i % 3), old = grid_of(*prob, ws, (i + 1) % 3);
+    a.w.gv = in.mm;
+    a.w.mm = out.mm;
+    a.w.flag = out.flag;
+    a.w.active = out.active;
+    const int ctas = persistent_ctas(prob, d->occ_g2p2g[0]);
+    launch_overlapped(par->actu ? k_g2p2g_rotate<128, true> : k_g2p2g_rotate<128, false>, ctas, 128, s, a, old,
+                      out.n_active);
     return cuda_ok();
 }
 
@@ -2894,9 +3116,22 @@ static int substeps_impl(const mpm_problem* prob, const mpm_tables* tab, mpm_par
     }
     if ((rc = launch_p2g(prob, tab, par, ws, s))) return rc;
     mark(MPM_KIND_P2G);
-    if ((rc = launch_grid_op(prob, tab, ws, s))) return rc;
-    mark(MPM_KIND_GRID_OP);
+    const bool rotate = !pr && rotate_applies(prob, tab);
+    int32_t k = 0;  // substeps since the last p2g
+    // the grid op that ends a stretch of substeps (before a re-sort, at the end)
+    auto grid_op = [&]() {
+        if (k == 0) return launch_grid_op(prob, tab, ws, s);
+        const Grid cur = grid_of(*prob, ws, k % 3), old = grid_of(*prob, ws, (k - 1) % 3);
+        return launch_grid_op(prob, tab, ws, s, true, &cur, &old);
+    };
     for (int32_t i = 1; i < n; ++i) {
+        if (!sort_due(i) && rotate) {
+            if ((rc = launch_rotate(prob, tab, par, ws, ++k, s))) return rc;
+            continue;
+        }
+        if ((rc = grid_op())) return rc;
+        k = 0;
+        mark(MPM_KIND_GRID_OP);
         if (sort_due(i)) {
             if ((rc = launch_g2p(prob, tab, par, ws, s))) return rc;
             mark(MPM_KIND_G2P);
@@ -2908,9 +3143,9 @@ static int substeps_impl(const mpm_problem* prob, const mpm_tables* tab, mpm_par
             if ((rc = launch_g2p2g(prob, tab, par, ws, s))) return rc;
             mark(MPM_KIND_G2P2G);
         }
-        if ((rc = launch_grid_op(prob, tab, ws, s))) return rc;
-        mark(MPM_KIND_GRID_OP);
     }
+    if ((rc = grid_op())) return rc;
+    mark(MPM_KIND_GRID_OP);
     if ((rc = launch_g2p(prob, tab, par, ws, s))) return rc;
     mark(MPM_KIND_G2P);
     return MPM_OK;
@@ -3007,6 +3242,9 @@ int mpm_substeps_noalloc(const mpm_problem* prob, const mpm_tables* tab, mpm_par
     if (rc) return rc;
     if ((rc = check_par(prob, par))) return rc;
     if (!tab || !tab->instances || !tab->materials || n_substeps < 0) return MPM_E_INVALID;
+    mpm_problem plain = *prob;  // the scratch holds no extra grids
+    plain.flags &= ~MPM_PROBF_ROTATE;
+    prob = &plain;
     const uint64_t need = layout_of(*prob).total;
     if (need > (uint64_t)MPM_NOALLOC_SCRATCH_BYTES) return MPM_E_CAPACITY;
     cudaStream_t s = (cudaStream_t)stream;
@@ -3025,6 +3263,9 @@ int mpm_noalloc_status(const mpm_problem* prob, int32_t clear, uint32_t* out, ui
     int rc = check_problem(prob);
     if (rc) return rc;
     if (!out) return MPM_E_INVALID;
+    mpm_problem plain = *prob;
+    plain.flags &= ~MPM_PROBF_ROTATE;
+    prob = &plain;
     if (layout_of(*prob).total > (uint64_t)MPM_NOALLOC_SCRATCH_BYTES) return MPM_E_CAPACITY;
     cudaStream_t s = (cudaStream_t)stream;
     void* ws = nullptr;

@@ -18,6 +18,12 @@ from .. import _native as nat
 
 F32_EPS = float(np.finfo(np.float32).eps)
 
+# Problems of up to this many particles get the two extra grids of MPM_PROBF_ROTATE, with which a run
+# of substeps folds the grid op into the particle kernel: 1.8x per substep at 1k particles, 1.07x at
+# 288k; the 500k scene, whose work items fill the GPU several times, ran 3% slower with it.
+ROTATE_MAX_PARTICLES = 300_000
+ROTATE_MAX_BYTES = 1 << 30  # of extra grids (32 bytes per node)
+
 
 @dataclass
 class InstanceSpec:
@@ -250,6 +256,12 @@ class MPMRuntime:
             cpic_normal=self.cpic_normal.data_ptr() if self.cpic_normal is not None else None,
             cpic_sep=self.cpic_sep.data_ptr() if self.cpic_sep is not None else None,
         )
+        # (a differentiated plastic rollout keeps the separate kernels: its gradient jumps where a return
+        # mapping switches branch, which another order of the grid's sums can cause)
+        plastic = any(m.kind in (nat.MAT_ELASTOPLASTIC, nat.MAT_SAND, nat.MAT_SNOW) for m in mats)
+        if (P == 128 and self.n <= ROTATE_MAX_PARTICLES and not colliders and not force_fields
+                and not (per_particle_lame and plastic) and 32 * 64 * self.n_blocks <= ROTATE_MAX_BYTES):
+            self.prob.flags |= nat.PROBF_ROTATE
         nbytes = C.c_uint64()
         nat.check("mpm_workspace_bytes", self.lib.mpm_workspace_bytes(C.byref(self.prob), C.byref(nbytes)))
         self.workspace_bytes = int(nbytes.value)

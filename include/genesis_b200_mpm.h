@@ -87,6 +87,9 @@ extern "C" {
 /* problem flags */
 #define MPM_PROBF_NONFREE 1      /* some particles are non-free: run the stencil-zeroing pass after p2g */
 #define MPM_PROBF_CPIC 2         /* CPIC against the colliders (mpm_particles.cpic_normal/cpic_sep required) */
+#define MPM_PROBF_ROTATE 4       /* the workspace holds two more grids (mpm_workspace_bytes counts them), and runs of
+                                    substeps fold the grid op into the particle kernel where nothing but gravity
+                                    and the boundary acts on the grid: for problems of up to some 10^5 particles */
 
 /* One simulated scene (one environment).  Mirrors the derived constants of
  * MPMSolver.__init__ (mpm_solver.py:31-78) and Simulator (simulator.py:110). */
