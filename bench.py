@@ -338,21 +338,27 @@ def kernel_breakdown(rt, n_substeps):
     total = sum(ms for ms, _ in prof.values())
     out = {}
     for k, (ms, launches) in prof.items():
-        groups = launches // (SORT_KERNELS if k == "sort" else 1)
+        groups = launches // (sort_kernels(rt) if k == "sort" else 1)
         if groups:
             out[k] = (ms / groups, groups, launches)
     return out, total
 
 
-SORT_KERNELS = 7  # keys, 3 scan passes, chunk table, scatter, lane deal
+def sort_kernels(rt):
+    """Kernels of one sort: keys, scan with the chunk table, scatter, lane deal; on grids of more
+    than 40,000 blocks 3 scan passes and the chunk table are kernels of their own."""
+    return 4 if rt.n_blocks <= 40000 else 7
 
 
-def launches_per_step(S, K):
+def launches_per_step(rt, S, K):
     """Kernel launches of one timed step (S substeps from a sort boundary): the runtime replays
     one CUDA graph per sort interval of K substeps, each the mpm_substeps schedule: the sort,
-    p2g and grid op, K - 1 times the fused g2p/p2g and the grid op, and the last g2p."""
+    p2g and grid op, K - 1 times the fused g2p/p2g and the grid op (one kernel where the runtime
+    folds the grid op into it), and the last g2p."""
+    from genesis_b200 import _native as nat
+
     graphs, rest = divmod(S, K)
-    per = lambda k: SORT_KERNELS + 2 + 2 * (k - 1) + 1
+    per = lambda k: sort_kernels(rt) + 2 + (1 if rt.prob.flags & nat.PROBF_ROTATE else 2) * (k - 1) + 1
     return graphs * per(K) + (per(rest) if rest else 0)
 
 
@@ -499,7 +505,7 @@ def run_ours(args, world, rank, local):
     # the committed ncu figure is the default scene's; other sizes report none
     traffic = tr.get(f"{dom}_dram_bytes_per_launch") if workload_name(args, d) == WORKLOAD else None
     sub_alg = SUBSTEP_BYTES[0] * d.n_particles + SUBSTEP_BYTES[1] * n_act
-    gpu_launches = args.steps * launches_per_step(S, args.sort_interval)
+    gpu_launches = args.steps * launches_per_step(rt, S, args.sort_interval)
 
     res = {
         "metric": METRIC,

@@ -505,19 +505,75 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_apply(int64_t nb, int P, Ws w) 
     }
 }
 
+// The scan and the chunk table of grids of up to kScanOneMax blocks in one CTA, a tile of bins at a
+// time with the totals carried along (65^3 nodes: two tiles; 129^3: nine), instead of four kernels.
+constexpr int64_t kScanOneMax = 40000;
+__global__ void __launch_bounds__(SCAN_T) k_scan_one(mpm_problem prob, const mpm_instance* __restrict__ inst, Ws w) {
+    __shared__ int2 s_warp[32];
+    pdl_wait();
+    pdl_trigger();
+    const int P = prob.chunk_particles;
+    const int nb = (int)prob.n_blocks;
+    int base_a = 0, base_c = 0;
+    for (int t0 = 0; t0 < nb; t0 += SCAN_TILE) {
+        const int j0 = t0 + (int)threadIdx.x * SCAN_ITEMS;
+        int va[SCAN_ITEMS], a = 0, c = 0;
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; ++i) {
+            va[i] = j0 + i < nb ? w.bin_count[j0 + i] : 0;
+            a += va[i];
+            c += (va[i] + P - 1) / P;
+        }
+        const int2 tot = block_exscan2(a, c, s_warp);
+        a += base_a;
+        c += base_c;
+        base_a += tot.x;
+        base_c += tot.y;
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; ++i) {
+            if (j0 + i < nb) w.bin_start[j0 + i] = a;
+            if (va[i] > 0) {
+                const int k = find_instance_by_block(inst, prob.n_instances, j0 + i);
+                const BlockCoord bc = block_coord((int)(j0 + i - inst[k].blk_base), inst[k]);
+                const int pbc = pack_bc(bc.bx, bc.by, bc.bz);
+                for (int s0 = a; s0 < a + va[i]; s0 += P)
+                    w.chunks[c++] = make_int4(k, pbc, s0, min(s0 + P, a + va[i]));
+            }
+            a += va[i];
+        }
+    }
+    if (threadIdx.x == 0) {
+        w.counters[CNT_CHUNKS] = (uint32_t)base_c;
+        w.counters[CNT_SORTED] = 1u;
+    }
+}
+
 __global__ void k_sort_scatter(mpm_problem prob, mpm_particles par, Ws w) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= prob.n_particles) return;
-    const int dst = w.bin_start[w.key[p]] + w.rank[p];
     const int64_t s = par.state_stride, t = w.tmp_stride;
-#pragma unroll 5
-    for (int ch = 0; ch < MPM_STATE_CH; ++ch) w.state_tmp[ch * t + dst] = par.state[ch * s + p];
-    w.mat_tmp[dst] = par.mat[p];
-    w.pflags_tmp[dst] = par.pflags[p];
-    w.gid_tmp[dst] = par.gid[p];
+    // every load in flight before the first store: a small problem has one or two warps per
+    // scheduler, and five rounds of load and store cost five L2 round trips
+    float v[MPM_STATE_CH], mu = 0.f, lam = 0.f;
+#pragma unroll
+    for (int ch = 0; ch < MPM_STATE_CH; ++ch) v[ch] = par.state[ch * s + p];
+    const uint8_t mat = par.mat[p], fl = par.pflags[p];
+    const int gid = par.gid[p], rank = w.rank[p], key = w.key[p];
     if (par.mu_p) {
-        w.mu_tmp[dst] = par.mu_p[p];
-        w.lam_tmp[dst] = par.lam_p[p];
+        mu = par.mu_p[p];
+        lam = par.lam_p[p];
+    }
+    pdl_wait();
+    pdl_trigger();
+    const int dst = w.bin_start[key] + rank;
+#pragma unroll
+    for (int ch = 0; ch < MPM_STATE_CH; ++ch) w.state_tmp[ch * t + dst] = v[ch];
+    w.mat_tmp[dst] = mat;
+    w.pflags_tmp[dst] = fl;
+    w.gid_tmp[dst] = gid;
+    if (par.mu_p) {
+        w.mu_tmp[dst] = mu;
+        w.lam_tmp[dst] = lam;
     }
 }
 
@@ -542,6 +598,7 @@ __global__ void __launch_bounds__(P) k_sort_interleave(mpm_problem prob, const m
                                                        mpm_particles par, Ws w) {
     __shared__ int cnt[32];
     __shared__ unsigned char s_slot[P];
+    pdl_wait();
     const int n_chunks = (int)w.counters[CNT_CHUNKS];
     const int64_t s = par.state_stride, t = w.tmp_stride;
     for (int ci = blockIdx.x; ci < n_chunks; ci += gridDim.x) {
@@ -552,13 +609,16 @@ __global__ void __launch_bounds__(P) k_sort_interleave(mpm_problem prob, const m
         const int n = ch.w - ch.z;
         const bool live = src < ch.w;
         int b = 0, r = 0;
+        float v[MPM_STATE_CH];  // (kept across the ordering: its loads overlap it)
         if (live) {
             const mpm_instance& I = inst[ch.x];
+#pragma unroll
+            for (int q = 0; q < MPM_STATE_CH; ++q) v[q] = w.state_tmp[q * t + src];
             int c[3];
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 // the cell of k_sort_keys, whose block is this chunk's block
-                const float f = floorf(w.state_tmp[(MPM_CH_X + d) * t + src] * I.inv_dx - 0.5f);
+                const float f = floorf(v[MPM_CH_X + d] * I.inv_dx - 0.5f);
                 const int cell = isfinite(f) ? (int)fminf(fmaxf(f - (float)I.lower_cell[d], 0.f), (float)(I.res[d] - 1)) : 0;
                 c[d] = cell & (BLK - 1);
             }
@@ -609,8 +669,8 @@ __global__ void __launch_bounds__(P) k_sort_interleave(mpm_problem prob, const m
                 pos = wb + (i & 3) * 8 + (i >> 2);
             }
             const int dst = ch.z + pos;
-#pragma unroll 5
-            for (int q = 0; q < MPM_STATE_CH; ++q) par.state[q * s + dst] = w.state_tmp[q * t + src];
+#pragma unroll
+            for (int q = 0; q < MPM_STATE_CH; ++q) par.state[q * s + dst] = v[q];
             par.mat[dst] = w.mat_tmp[src];
             par.pflags[dst] = w.pflags_tmp[src];
             const int g = w.gid_tmp[src];
@@ -2426,23 +2486,27 @@ static int launch_sort(const mpm_problem* prob, const mpm_tables* tab, mpm_parti
     const int T = 256;
     if (n > 0) k_sort_keys<<<(n + T - 1) / T, T, 0, s>>>(*prob, tab->instances, *par, w);
     const int ntiles = (int)((nb + SCAN_TILE - 1) / SCAN_TILE);
-    k_scan_reduce<<<ntiles, SCAN_T, 0, s>>>(nb, prob->chunk_particles, w);
-    k_scan_tiles<<<1, SCAN_T, 0, s>>>(ntiles, w);
-    k_scan_apply<<<ntiles, SCAN_T, 0, s>>>(nb, prob->chunk_particles, w);
-    k_build_chunks<<<(int)((nb + T - 1) / T), T, 0, s>>>(*prob, tab->instances, w);
+    if (nb <= kScanOneMax && n > 0) {
+        launch_overlapped(k_scan_one, 1, SCAN_T, s, *prob, tab->instances, w);
+    } else {
+        k_scan_reduce<<<ntiles, SCAN_T, 0, s>>>(nb, prob->chunk_particles, w);
+        k_scan_tiles<<<1, SCAN_T, 0, s>>>(ntiles, w);
+        k_scan_apply<<<ntiles, SCAN_T, 0, s>>>(nb, prob->chunk_particles, w);
+        k_build_chunks<<<(int)((nb + T - 1) / T), T, 0, s>>>(*prob, tab->instances, w);
+    }
     if (n > 0) {
-        k_sort_scatter<<<(n + T - 1) / T, T, 0, s>>>(*prob, *par, w);
+        launch_overlapped(k_sort_scatter, (n + T - 1) / T, T, s, *prob, *par, w);
         const DevInfo* d = dev_info();
         if (!d) return MPM_E_CUDA;
         const int P = prob->chunk_particles;
         int ctas = d->sms * (2048 / P);
         if (ctas > prob->max_chunks) ctas = prob->max_chunks > 0 ? prob->max_chunks : 1;
         if (P == 128)
-            k_sort_interleave<128><<<ctas, 128, 0, s>>>(*prob, tab->instances, *par, w);
+            launch_overlapped(k_sort_interleave<128>, ctas, 128, s, *prob, tab->instances, *par, w);
         else if (P == 256)
-            k_sort_interleave<256><<<ctas, 256, 0, s>>>(*prob, tab->instances, *par, w);
+            launch_overlapped(k_sort_interleave<256>, ctas, 256, s, *prob, tab->instances, *par, w);
         else
-            k_sort_interleave<512><<<ctas, 512, 0, s>>>(*prob, tab->instances, *par, w);
+            launch_overlapped(k_sort_interleave<512>, ctas, 512, s, *prob, tab->instances, *par, w);
     }
     return cuda_ok();
 }
@@ -3175,8 +3239,10 @@ int mpm_substeps_profile(const mpm_problem* prob, const mpm_tables* tab, mpm_par
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, pr.ev[i - 1], pr.ev[i]) != cudaSuccess) return MPM_E_CUDA;
         ms_by_kind[pr.kind[i]] += ms;
-        // a sort is 7 kernels (keys, 3 scan passes, chunk table, scatter, lane deal), 4 without particles
-        launches_by_kind[pr.kind[i]] += pr.kind[i] == MPM_KIND_SORT ? (prob->n_particles > 0 ? 7 : 4) : 1;
+        // a sort is 4 kernels (keys, scan with the chunk table, scatter, lane deal), or 7 on large grids (3
+        // scan passes, the chunk table by itself), 4 of them without particles
+        const int sort_kernels = prob->n_particles > 0 && prob->n_blocks > kScanOneMax ? 7 : 4;
+        launches_by_kind[pr.kind[i]] += pr.kind[i] == MPM_KIND_SORT ? sort_kernels : 1;
     }
     return MPM_OK;
 }
