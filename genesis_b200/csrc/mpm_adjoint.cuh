@@ -70,77 +70,102 @@ __device__ __forceinline__ bool node_ok(const mpm_instance& I, int gx, int gy, i
 }
 
 // ---- adjoint of g2p (mpm_solver.py:396-437)
+// Bound: latency.  A differentiable scene of some 10^4 particles is one CTA per SM, and the three
+// adjoint kernels of a substep depend on one another, so what counts is the chain through them.  In
+// the recorded reverse pass they are launched to overlap: each does all that the records alone
+// determine (here the gathered velocity, in k_adj_p2g the SVD and the stress) before pdl_wait(),
+// beside the kernels before it.  The outermost stencil loops are rolled: nine nodes' loads in flight
+// at a time and a third of the code, whose fetch a lone warp per scheduler waits for.
+// The three kernels of a 20k-particle substep, replayed alone: 34.7 us (52 us one after the other).
 __global__ void k_adj_g2p(mpm_problem prob, const mpm_instance* __restrict__ inst, mpm_particles par, float* adj,
                           Ws w, AdjWs aw) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= prob.n_particles || !(par.pflags[s] & MPM_PFLAG_ACTIVE)) return;
-    const mpm_instance& I = inst[find_instance_by_particle(inst, prob.n_instances, s)];
     const int64_t st = par.state_stride;
-    float x[3], fx[3], wv[3][3], dwv[3][3];
+    float x[3] = {0.f, 0.f, 0.f}, fx[3], wv[3][3], dwv[3][3], nv[3] = {0.f, 0.f, 0.f};
     int base[3];
+    bool live = s < prob.n_particles && (par.pflags[s] & MPM_PFLAG_ACTIVE);
+    const mpm_instance& I = inst[live ? find_instance_by_particle(inst, prob.n_instances, s) : 0];
+    if (live) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) x[d] = par.state[(MPM_CH_X + d) * st + s];
-    if (!finite3(x[0], x[1], x[2])) return;
-    locate(I, x, base, fx);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) bspline_d(fx[d], wv[d], dwv[d]);
-    // recompute the gathered velocity for the boundary masks.  The 27 node velocities are
-    // loaded once, all issued before the first is used (one CTA per SM at the differentiable
-    // scenes' sizes: the loads' latency, not bandwidth, sets this kernel's time), and kept in
-    // registers for the scatter below.
-    float4 gn[27];
-#pragma unroll
-    for (int n = 0; n < 27; ++n) {
-        const int gx = base[0] + n / 9, gy = base[1] + (n / 3) % 3, gz = base[2] + n % 3;
-        gn[n] = node_ok(I, gx, gy, gz) ? w.gv[node_addr(I, gx, gy, gz)] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int d = 0; d < 3; ++d) x[d] = par.state[(MPM_CH_X + d) * st + s];
+        live = finite3(x[0], x[1], x[2]);
     }
-    float nv[3] = {0.f, 0.f, 0.f};
+    if (live) {
+        locate(I, x, base, fx);
 #pragma unroll
-    for (int n = 0; n < 27; ++n) {
-        const float wt = wv[0][n / 9] * wv[1][(n / 3) % 3] * wv[2][n % 3];
-        nv[0] += wt * gn[n].x;
-        nv[1] += wt * gn[n].y;
-        nv[2] += wt * gn[n].z;
+        for (int d = 0; d < 3; ++d) bspline_d(fx[d], wv[d], dwv[d]);
+        // recompute the gathered velocity for the boundary masks
+#pragma unroll 1
+        for (int i = 0; i < 3; ++i) {
+            float4 g[9];
+#pragma unroll
+            for (int n = 0; n < 9; ++n) {
+                const int gx = base[0] + i, gy = base[1] + n / 3, gz = base[2] + n % 3;
+                g[n] = node_ok(I, gx, gy, gz) ? w.gv[node_addr(I, gx, gy, gz)] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            const float wi = sel3(wv[0], i);
+#pragma unroll
+            for (int n = 0; n < 9; ++n) {
+                const float wt = wi * wv[1][n / 3] * wv[2][n % 3];
+                nv[0] += wt * g[n].x;
+                nv[1] += wt * g[n].y;
+                nv[2] += wt * g[n].z;
+            }
+        }
     }
+    pdl_wait();
+    pdl_trigger();
+    if (!live) return;
     float gxb[3], vb[3], Cb[9];
     const float* xin = adj + (int64_t)MPM_CH_X * st;
     const float* vin = adj + (int64_t)MPM_CH_V * st;
     const float* cin = adj + (int64_t)MPM_CH_C * st;
 #pragma unroll
+    for (int k = 0; k < 9; ++k) Cb[k] = cin[k * st + s];
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
         const float xs = x[d] + I.dt * nv[d];
         const bool clamped = xs > I.bnd_hi[d] || xs < I.bnd_lo[d];
         const bool vzero = (xs >= I.bnd_hi[d] && nv[d] >= 0.f) || (xs <= I.bnd_lo[d] && nv[d] <= 0.f);
-        gxb[d] = clamped ? 0.f : xin[d * st + s];
-        vb[d] = (vzero ? 0.f : vin[d * st + s]) + I.dt * gxb[d];
+        const float xi = xin[d * st + s], vi = vin[d * st + s];
+        gxb[d] = clamped ? 0.f : xi;
+        vb[d] = (vzero ? 0.f : vi) + I.dt * gxb[d];
     }
-#pragma unroll
-    for (int k = 0; k < 9; ++k) Cb[k] = cin[k * st + s];
     float xb[3] = {gxb[0], gxb[1], gxb[2]};
     const float c = I.c_scale;
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+        const float wi = sel3(wv[0], i), dwi = sel3(dwv[0], i);
+        float4 g[9];
 #pragma unroll
-    for (int n = 0; n < 27; ++n) {
-        const int i = n / 9, j = (n / 3) % 3, k = n % 3;
-        const int gx = base[0] + i, gy = base[1] + j, gz = base[2] + k;
-        if (!node_ok(I, gx, gy, gz)) continue;
-        const int64_t na = node_addr(I, gx, gy, gz);
-        const float vh[3] = {gn[n].x, gn[n].y, gn[n].z};
-        const float wt = wv[0][i] * wv[1][j] * wv[2][k];
-        const float gw[3] = {dwv[0][i] * wv[1][j] * wv[2][k] * I.inv_dx, wv[0][i] * dwv[1][j] * wv[2][k] * I.inv_dx,
-                             wv[0][i] * wv[1][j] * dwv[2][k] * I.inv_dx};
-        const float u[3] = {(float)i - fx[0], (float)j - fx[1], (float)k - fx[2]};
-        float Cu[3];
+        for (int n = 0; n < 9; ++n) {
+            const int gx = base[0] + i, gy = base[1] + n / 3, gz = base[2] + n % 3;
+            g[n] = node_ok(I, gx, gy, gz) ? w.gv[node_addr(I, gx, gy, gz)] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
 #pragma unroll
-        for (int a = 0; a < 3; ++a) Cu[a] = Cb[a * 3 + 0] * u[0] + Cb[a * 3 + 1] * u[1] + Cb[a * 3 + 2] * u[2];
-        // one 16-byte vector reduction per node (sm_90+) instead of three scalar ones
-        atomicAdd(&aw.vbar[na], make_float4(wt * vb[0] + c * wt * Cu[0], wt * vb[1] + c * wt * Cu[1],
-                                            wt * vb[2] + c * wt * Cu[2], 0.f));
-        const float wbar = vb[0] * vh[0] + vb[1] * vh[1] + vb[2] * vh[2] +
-                           c * (vh[0] * Cu[0] + vh[1] * Cu[1] + vh[2] * Cu[2]);
+        for (int n = 0; n < 9; ++n) {
+            const int j = n / 3, k = n % 3;
+            const int gx = base[0] + i, gy = base[1] + j, gz = base[2] + k;
+            if (!node_ok(I, gx, gy, gz)) continue;
+            const float vh[3] = {g[n].x, g[n].y, g[n].z};
+            const float wt = wi * wv[1][j] * wv[2][k];
+            const float gw[3] = {dwi * wv[1][j] * wv[2][k] * I.inv_dx, wi * dwv[1][j] * wv[2][k] * I.inv_dx,
+                                 wi * wv[1][j] * dwv[2][k] * I.inv_dx};
+            const float u[3] = {(float)i - fx[0], (float)j - fx[1], (float)k - fx[2]};
+            float Cu[3];
 #pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            const float ub = c * wt * (Cb[0 * 3 + e] * vh[0] + Cb[1 * 3 + e] * vh[1] + Cb[2 * 3 + e] * vh[2]);
-            xb[e] += wbar * gw[e] - I.inv_dx * ub;
+            for (int a = 0; a < 3; ++a) Cu[a] = Cb[a * 3 + 0] * u[0] + Cb[a * 3 + 1] * u[1] + Cb[a * 3 + 2] * u[2];
+            // one 16-byte vector reduction per node (sm_90+) instead of three scalar ones
+            atomicAdd(&aw.vbar[node_addr(I, gx, gy, gz)],
+                      make_float4(wt * vb[0] + c * wt * Cu[0], wt * vb[1] + c * wt * Cu[1],
+                                  wt * vb[2] + c * wt * Cu[2], 0.f));
+            const float wbar = vb[0] * vh[0] + vb[1] * vh[1] + vb[2] * vh[2] +
+                               c * (vh[0] * Cu[0] + vh[1] * Cu[1] + vh[2] * Cu[2]);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                const float ub = c * wt * (Cb[0 * 3 + e] * vh[0] + Cb[1 * 3 + e] * vh[1] + Cb[2 * 3 + e] * vh[2]);
+                xb[e] += wbar * gw[e] - I.inv_dx * ub;
+            }
         }
     }
 #pragma unroll
@@ -504,10 +529,14 @@ __global__ void __launch_bounds__(256) k_adj_grid_active(mpm_problem prob, const
                                                          const uint32_t* __restrict__ n_active_p,
                                                          const mpm_force_field* __restrict__ ffs, int n_ff,
                                                          const int* __restrict__ ff_perm) {
+    // before the wait already: the next kernel's prologue reads only the records and what the kernels
+    // before this one's predecessor wrote, which had completed when this one could start
+    pdl_trigger();
     const int n_active = (int)*n_active_p;
     const int gpc = blockDim.x / BLK3;
     const int grp = threadIdx.x / BLK3;
     const int ln = threadIdx.x % BLK3;
+    pdl_wait();
     const int lxyz[3] = {ln / (BLK * BLK), (ln / BLK) % BLK, ln % BLK};
     for (int i = blockIdx.x * gpc + grp; i < n_active; i += gridDim.x * gpc) {
         const int2 e = active[i];
@@ -908,7 +937,10 @@ __global__ void k_adj_p2g(mpm_problem prob, const mpm_instance* __restrict__ ins
                           const mpm_material* __restrict__ mats, mpm_particles par, float* adj, float* lame_bar,
                           AdjWs aw) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= prob.n_particles || !(par.pflags[s] & MPM_PFLAG_ACTIVE)) return;
+    if (s >= prob.n_particles || !(par.pflags[s] & MPM_PFLAG_ACTIVE)) {
+        pdl_wait();
+        return;
+    }
     const mpm_instance& I = inst[find_instance_by_particle(inst, prob.n_instances, s)];
     const mpm_material m = mats[I.mat_base + par.mat[s]];
     const int64_t st = par.state_stride;
@@ -924,7 +956,18 @@ __global__ void k_adj_p2g(mpm_problem prob, const mpm_instance* __restrict__ ins
         C[k] = S[(MPM_CH_C + k) * st + s];
         F[k] = S[(MPM_CH_F + k) * st + s];
     }
-    if (!finite3(x[0], x[1], x[2])) return;
+    if (!finite3(x[0], x[1], x[2])) {
+        pdl_wait();
+        return;
+    }
+    // (adj's F and Jp rows were last written by this kernel for the substep after, two kernels before
+    // the one it waits for)
+    float* fo = adj + (int64_t)MPM_CH_F * st;
+    float* jo = adj + (int64_t)MPM_CH_JP * st;
+    float Gb[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Gb[k] = __ldcg(&fo[k * st + s]);
+    const float Jpnb = __ldcg(&jo[s]);
     const float mu = par.mu_p ? ((m.kind == MPM_MAT_LIQUID && m.mu == 0.f) ? 0.f : par.mu_p[s]) : m.mu;
     const float lam = par.lam_p ? par.lam_p[s] : m.lam;
     // forward recompute
@@ -969,35 +1012,45 @@ __global__ void k_adj_p2g(mpm_problem prob, const mpm_instance* __restrict__ ins
     locate(I, x, base, fx);
 #pragma unroll
     for (int d = 0; d < 3; ++d) bspline_d(fx[d], wv[d], dwv[d]);
+    pdl_wait();
+    pdl_trigger();
     // adjoint of the scatter
     float xb[3] = {aw.xbar[0 * aw.stride + s], aw.xbar[1 * aw.stride + s], aw.xbar[2 * aw.stride + s]};
     float vbn[3] = {0.f, 0.f, 0.f};
     float Ab[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const float dx = I.dx;
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j)
-            for (int k = 0; k < 3; ++k) {
-                const int gx = base[0] + i, gy = base[1] + j, gz = base[2] + k;
-                if (!node_ok(I, gx, gy, gz)) continue;
-                const float4 pmb = aw.pmbar[node_addr(I, gx, gy, gz)];
-                const float pb[3] = {pmb.x, pmb.y, pmb.z};
-                const float wt = wv[0][i] * wv[1][j] * wv[2][k];
-                const float gw[3] = {dwv[0][i] * wv[1][j] * wv[2][k] * I.inv_dx, wv[0][i] * dwv[1][j] * wv[2][k] * I.inv_dx,
-                                     wv[0][i] * wv[1][j] * dwv[2][k] * I.inv_dx};
-                const float d[3] = {((float)i - fx[0]) * dx, ((float)j - fx[1]) * dx, ((float)k - fx[2]) * dx};
-                float wbar = pmb.w * mass;
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+        const float wi = sel3(wv[0], i), dwi = sel3(dwv[0], i);
+        float4 pm[9];
 #pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const float q = mass * v[a] + A[a * 3 + 0] * d[0] + A[a * 3 + 1] * d[1] + A[a * 3 + 2] * d[2];
-                    wbar += pb[a] * q;
-                    vbn[a] += wt * mass * pb[a];
+        for (int n = 0; n < 9; ++n) {
+            const int gx = base[0] + i, gy = base[1] + n / 3, gz = base[2] + n % 3;
+            pm[n] = node_ok(I, gx, gy, gz) ? aw.pmbar[node_addr(I, gx, gy, gz)] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
 #pragma unroll
-                    for (int b = 0; b < 3; ++b) Ab[a * 3 + b] += wt * pb[a] * d[b];
-                }
+        for (int n = 0; n < 9; ++n) {
+            const int j = n / 3, k = n % 3;
+            if (!node_ok(I, base[0] + i, base[1] + j, base[2] + k)) continue;
+            const float pb[3] = {pm[n].x, pm[n].y, pm[n].z};
+            const float wt = wi * wv[1][j] * wv[2][k];
+            const float gw[3] = {dwi * wv[1][j] * wv[2][k] * I.inv_dx, wi * dwv[1][j] * wv[2][k] * I.inv_dx,
+                                 wi * wv[1][j] * dwv[2][k] * I.inv_dx};
+            const float d[3] = {((float)i - fx[0]) * dx, ((float)j - fx[1]) * dx, ((float)k - fx[2]) * dx};
+            float wbar = pm[n].w * mass;
 #pragma unroll
-                for (int e = 0; e < 3; ++e)
-                    xb[e] += wbar * gw[e] - wt * (A[0 * 3 + e] * pb[0] + A[1 * 3 + e] * pb[1] + A[2 * 3 + e] * pb[2]);
+            for (int a = 0; a < 3; ++a) {
+                const float q = mass * v[a] + A[a * 3 + 0] * d[0] + A[a * 3 + 1] * d[1] + A[a * 3 + 2] * d[2];
+                wbar += pb[a] * q;
+                vbn[a] += wt * mass * pb[a];
+#pragma unroll
+                for (int b = 0; b < 3; ++b) Ab[a * 3 + b] += wt * pb[a] * d[b];
             }
+#pragma unroll
+            for (int e = 0; e < 3; ++e)
+                xb[e] += wbar * gw[e] - wt * (A[0 * 3 + e] * pb[0] + A[1 * 3 + e] * pb[1] + A[2 * 3 + e] * pb[2]);
+        }
+    }
     // A = s P + m C
     float Pb[9], Cbn[9];
 #pragma unroll
@@ -1032,13 +1085,8 @@ __global__ void k_adj_p2g(mpm_problem prob, const mpm_instance* __restrict__ ins
     float* xo = adj + (int64_t)MPM_CH_X * st;
     float* vo = adj + (int64_t)MPM_CH_V * st;
     float* co = adj + (int64_t)MPM_CH_C * st;
-    float* fo = adj + (int64_t)MPM_CH_F * st;
-    float* jo = adj + (int64_t)MPM_CH_JP * st;
-    float Gb[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) Gb[k] = fo[k * st + s];
     float Jpb = 0.f;
-    material_adjoint(m, mu, lam, I.eps, U, Sg, V, Jp, Gb, jo[s], Pb, Ftb, Jpb, mub, lamb);
+    material_adjoint(m, mu, lam, I.eps, U, Sg, V, Jp, Gb, Jpnb, Pb, Ftb, Jpb, mub, lamb);
     // F_tmp = (I + dt C) F
     float Fbn[9];
 #pragma unroll

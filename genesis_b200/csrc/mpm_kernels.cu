@@ -1525,8 +1525,24 @@ __device__ __forceinline__ void scatter_flush(Tile& T, const Payload& o, const m
             }
             }
         } else {
-            // drifted since the last sort (or a non-finite stress): bounds-checked global path
+            // drifted since the last sort (or a non-finite stress): bounds-checked global path.  The
+            // blocks it reaches are marked first, each once: a flag read per node was 27 L2 round trips
+            // that the whole CTA waited for
             atomicAdd((unsigned long long*)&w.counters[CNT_FALLBACK], 1ull);
+            {
+                int lo[3], hi[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    lo[d] = max(o.base[d], 0) >> 2;
+                    hi[d] = o.base[d] > I.res[d] - 1 ? -1 : min(o.base[d] + 2, I.res[d] - 1) >> 2;
+                }
+#pragma unroll 1
+                for (int bx = lo[0]; bx <= hi[0]; ++bx)
+#pragma unroll 1
+                    for (int by = lo[1]; by <= hi[1]; ++by)
+#pragma unroll 1
+                        for (int bz = lo[2]; bz <= hi[2]; ++bz) mark_block(w, inst, I, bx, by, bz, n_active);
+            }
 #pragma unroll 1
             for (int i = 0; i < 3; ++i)
 #pragma unroll 1
@@ -1551,7 +1567,6 @@ __device__ __forceinline__ void scatter_flush(Tile& T, const Payload& o, const m
                         const float ay = o.q[1] + (o.A[3] * i + o.A[4] * j + o.A[5] * k);
                         const float az = o.q[2] + (o.A[6] * i + o.A[7] * j + o.A[8] * k);
                         atomicAdd(&w.mm[node_addr(I, gx, gy, gz)], make_float4(wt * ax, wt * ay, wt * az, wt * o.mass));
-                        mark_block(w, inst, I, gx >> 2, gy >> 2, gz >> 2, n_active);
                     }
         }
     }
@@ -1737,16 +1752,22 @@ __device__ __forceinline__ bool gather(const VelTile& VT, const Ws& w, const mpm
 #pragma unroll 1
         for (int i = 0; i < 3; ++i)
 #pragma unroll 1
-            for (int j = 0; j < 3; ++j)
-#pragma unroll 1
+            for (int j = 0; j < 3; ++j) {
+                // the three nodes' loads in flight together (one at a time was 27 L2 round trips)
+                float4 gk[3];
+                bool ok[3];
+#pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     const int gx = base[0] + i, gy = base[1] + j, gz = base[2] + k;
-                    if (gx < 0 || gy < 0 || gz < 0 || gx >= I.res[0] || gy >= I.res[1] || gz >= I.res[2]) {
-                        set_status(w, inst, MPM_STATUS_OUT_OF_GRID);
-                        continue;
-                    }
-                    float4 g = w.gv[node_addr(I, gx, gy, gz)];
-                    if constexpr (RAW) g = node_velocity(I, g, gx, gy, gz);
+                    ok[k] = !(gx < 0 || gy < 0 || gz < 0 || gx >= I.res[0] || gy >= I.res[1] || gz >= I.res[2]);
+                    gk[k] = ok[k] ? w.gv[node_addr(I, gx, gy, gz)] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (!ok[k]) set_status(w, inst, MPM_STATUS_OUT_OF_GRID);
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    if (!ok[k]) continue;
+                    float4 g = gk[k];
+                    if constexpr (RAW) g = node_velocity(I, g, base[0] + i, base[1] + j, base[2] + k);
                     const float wt = sel3(wx, i) * sel3(wy, j) * sel3(wz, k);
                     const float d0 = (float)i - fx[0], d1 = (float)j - fx[1], d2 = (float)k - fx[2];
                     nv[0] += wt * g.x;
@@ -1763,6 +1784,7 @@ __device__ __forceinline__ bool gather(const VelTile& VT, const Ws& w, const mpm
                     nC[7] += cw * g.z * d1;
                     nC[8] += cw * g.z * d2;
                 }
+            }
     }
     if constexpr (CPIC)
         cpic_correct(*cp, &VT, w, I, p, x, base, fx, wx, wy, wz, tile_contains(base, ox, oy, oz), ox, oy, oz, nv, nC);
@@ -2233,16 +2255,28 @@ __device__ __forceinline__ void apply_force_fields(const mpm_force_field* __rest
     }
 }
 
+// One recorded substep of grid_rec: the momentum and mass after p2g and the velocity after
+// the grid op (float4 per node each), then the active-block list the grid op walked and its
+// length.
+struct RecGrid {
+    float4* mm;
+    float4* gv;
+    int2* active;
+    uint32_t* n_active;
+};
+
 // at most 64 registers (4 CTAs per SM): the collider responses, rare, may spill instead.
 // FF: the problem has force fields (a separate instantiation keeps their registers out of
-// the common path)
-template <bool FF>
+// the common path).  REC: the substep is recorded for the reverse pass: the active list, and each
+// node's momentum, mass and velocity (two kernels of their own before, a copy before and after)
+template <bool FF, bool REC = false>
 __global__ void __launch_bounds__(256, 4) k_grid_op(mpm_problem prob, const mpm_instance* __restrict__ inst, Ws w,
                                                  const mpm_collider* __restrict__ colliders, int n_colliders,
                                                  float* collider_force, const float* __restrict__ sdf_voxels,
                                                  const mpm_force_field* __restrict__ ffs, int n_ff,
-                                                 const int* __restrict__ ff_perm, int count_op, uint32_t* count, Grid old) {
+                                                 const int* __restrict__ ff_perm, int count_op, uint32_t* count, Grid old, RecGrid rec) {
     const int n_active = (int)*count;
+    if (REC && blockIdx.x == 0 && threadIdx.x == 0) *rec.n_active = (uint32_t)n_active;
     const uint32_t ops = w.counters[CNT_GRID_OPS];
     const int gpc = blockDim.x / BLK3;
     const int grp = threadIdx.x / BLK3;
@@ -2297,6 +2331,11 @@ __global__ void __launch_bounds__(256, 4) k_grid_op(mpm_problem prob, const mpm_
             vz = bc_vel(pz, vz, I.bnd_lo[2], I.bnd_hi[2]);
         }
         w.gv[g] = make_float4(vx, vy, vz, vz);  // w: a copy of z for the packed gather
+        if (REC) {
+            rec.mm[g] = mm;
+            rec.gv[g] = make_float4(vx, vy, vz, vz);
+            if (ln == 0) rec.active[i] = e;
+        }
         w.mm[g] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (ln == 0) w.flag[I.blk_base + lb] = 0u;
     }
@@ -2575,7 +2614,8 @@ static int launch_p2g(const mpm_problem* prob, const mpm_tables* tab, mpm_partic
 // advance = false (the adjoint's recompute): the colliders keep their pose and accumulate no force
 // cur, old: the grids that a rotating run ends with (the one to update, the one to clear)
 static int launch_grid_op(const mpm_problem* prob, const mpm_tables* tab, void* ws, cudaStream_t s,
-                          bool advance = true, const Grid* cur = nullptr, const Grid* old = nullptr) {
+                          bool advance = true, const Grid* cur = nullptr, const Grid* old = nullptr,
+                          const RecGrid* rec = nullptr) {
     const DevInfo* d = dev_info();
     if (!d) return MPM_E_CUDA;
     int ctas = prob->grid_ctas > 0 ? prob->grid_ctas : d->sms * d->occ_grid;
@@ -2594,14 +2634,11 @@ static int launch_grid_op(const mpm_problem* prob, const mpm_tables* tab, void* 
         count = cur->n_active;
     }
     const Grid none{nullptr, nullptr, nullptr, nullptr};
-    if (nff > 0)
-        k_grid_op<true><<<ctas, 256, 0, s>>>(*prob, tab->instances, w, tab->colliders, nc,
-                                              advance ? tab->collider_force : nullptr, tab->sdf_voxels,
-                                              tab->force_fields, nff, tab->ff_perm, advance ? 1 : 0, count, none);
-    else
-        k_grid_op<false><<<ctas, 256, 0, s>>>(*prob, tab->instances, w, tab->colliders, nc,
-                                               advance ? tab->collider_force : nullptr, tab->sdf_voxels, nullptr, 0,
-                                               nullptr, advance ? 1 : 0, count, old ? *old : none);
+    auto* k = nff > 0 ? (rec ? k_grid_op<true, true> : k_grid_op<true, false>)
+                      : (rec ? k_grid_op<false, true> : k_grid_op<false, false>);
+    k<<<ctas, 256, 0, s>>>(*prob, tab->instances, w, tab->colliders, nc, advance ? tab->collider_force : nullptr,
+                           tab->sdf_voxels, nff > 0 ? tab->force_fields : nullptr, nff, nff > 0 ? tab->ff_perm : nullptr,
+                           advance ? 1 : 0, count, old ? *old : none, rec ? *rec : RecGrid{});
     if (nc > 0 && advance)
         k_advance_colliders<<<(nc + 63) / 64, 64, 0, s>>>(tab->instances, prob->n_instances, tab->colliders, nc);
     return cuda_ok();
@@ -3400,16 +3437,6 @@ int mpm_substep_adjoint_colliders(const mpm_problem* prob, const mpm_tables* tab
     return cuda_ok();
 }
 
-// One recorded substep of grid_rec: the momentum and mass after p2g and the velocity after
-// the grid op (float4 per node each), then the active-block list the grid op walked and its
-// length.
-struct RecGrid {
-    float4* mm;
-    float4* gv;
-    int2* active;
-    uint32_t* n_active;
-};
-
 static uint64_t rec_grid_bytes(const mpm_problem& p) {
     const uint64_t nodes = (uint64_t)p.n_blocks * BLK3;
     return align_up(nodes * 32 + (uint64_t)p.n_blocks * 8 + 16, 256);
@@ -3424,37 +3451,6 @@ static RecGrid rec_grid_of(const mpm_problem& p, void* base, int32_t j) {
     r.active = (int2*)(b + nodes * 32);
     r.n_active = (uint32_t*)(b + nodes * 32 + (uint64_t)p.n_blocks * 8);
     return r;
-}
-
-// Record the p2g result of the active blocks: their list, its length and their momentum and
-// mass (the grid op, which runs next, clears both behind itself).  One 64-thread group per
-// block; the adjoint reads nothing outside the active blocks.
-__device__ __forceinline__ int64_t block_of_entry(const mpm_instance* __restrict__ inst, int2 e) {
-    const mpm_instance& I = inst[e.x];
-    const BlockCoord bc = unpack_bc(e.y);
-    return I.blk_base + local_block(I, bc.bx, bc.by, bc.bz);
-}
-
-__global__ void __launch_bounds__(256) k_record_p2g(const mpm_instance* __restrict__ inst, Ws w, RecGrid r) {
-    const int n_active = (int)w.counters[CNT_ACTIVE];
-    const int gpc = blockDim.x / BLK3, grp = threadIdx.x / BLK3, ln = threadIdx.x % BLK3;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *r.n_active = (uint32_t)n_active;
-    for (int i = blockIdx.x * gpc + grp; i < n_active; i += gridDim.x * gpc) {
-        const int2 e = w.active[i];
-        if (ln == 0) r.active[i] = e;
-        const int64_t blk = block_of_entry(inst, e);
-        r.mm[blk * BLK3 + ln] = w.mm[blk * BLK3 + ln];
-    }
-}
-
-// Record the grid op's velocity of the blocks k_record_p2g listed.
-__global__ void __launch_bounds__(256) k_record_gv(const mpm_instance* __restrict__ inst, Ws w, RecGrid r) {
-    const int n_active = (int)*r.n_active;
-    const int gpc = blockDim.x / BLK3, grp = threadIdx.x / BLK3, ln = threadIdx.x % BLK3;
-    for (int i = blockIdx.x * gpc + grp; i < n_active; i += gridDim.x * gpc) {
-        const int64_t blk = block_of_entry(inst, r.active[i]);
-        r.gv[blk * BLK3 + ln] = w.gv[blk * BLK3 + ln];
-    }
 }
 
 int mpm_record_grid_bytes(const mpm_problem* prob, uint64_t* out) {
@@ -3475,23 +3471,13 @@ int mpm_substeps_record(const mpm_problem* prob, const mpm_tables* tab, mpm_part
     if (n_substeps > 0 && (!state_rec || !grid_rec)) return MPM_E_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t plane = (size_t)MPM_STATE_CH * (size_t)par->state_stride;  // floats per recorded state
-    Ws w = ws_of(*prob, workspace);
-    const DevInfo* d = dev_info();
-    if (!d) return MPM_E_CUDA;
-    int rctas = d->sms * 4;
-    const int64_t need = (prob->n_blocks + 3) / 4;
-    if (rctas > need) rctas = (int)(need > 0 ? need : 1);
     for (int32_t j = 0; j < n_substeps; ++j) {
         const RecGrid r = rec_grid_of(*prob, grid_rec, j);
         if (cudaMemcpyAsync(state_rec + (size_t)j * plane, par->state, plane * 4, cudaMemcpyDeviceToDevice, s) !=
             cudaSuccess)
             return MPM_E_CUDA;
         if ((rc = launch_p2g(prob, tab, par, workspace, s))) return rc;
-        // the grid op clears the momentum behind itself and resets the active count: keep the
-        // p2g result and the list first
-        k_record_p2g<<<rctas, 256, 0, s>>>(tab->instances, w, r);
-        if ((rc = launch_grid_op(prob, tab, workspace, s))) return rc;
-        k_record_gv<<<rctas, 256, 0, s>>>(tab->instances, w, r);
+        if ((rc = launch_grid_op(prob, tab, workspace, s, true, nullptr, nullptr, &r))) return rc;
         if ((rc = launch_g2p(prob, tab, par, workspace, s))) return rc;
     }
     return cuda_ok();
@@ -3530,10 +3516,11 @@ int mpm_substeps_adjoint_recorded(const mpm_problem* prob, const mpm_tables* tab
         aw.saved_mm = r.mm;
         w.gv = r.gv;
         if (n > 0) {
-            k_adj_g2p<<<(n + 127) / 128, 128, 0, s>>>(*prob, tab->instances, sp, adj, w, aw);
-            k_adj_grid_active<<<gctas, 256, 0, s>>>(*prob, tab->instances, aw, r.active, r.n_active, tab->force_fields,
-                                                    nff, tab->ff_perm);
-            k_adj_p2g<<<(n + 127) / 128, 128, 0, s>>>(*prob, tab->instances, tab->materials, sp, adj, lame_bar, aw);
+            launch_overlapped(k_adj_g2p, (n + 127) / 128, 128, s, *prob, tab->instances, sp, adj, w, aw);
+            launch_overlapped(k_adj_grid_active, gctas, 256, s, *prob, tab->instances, aw, r.active, r.n_active,
+                              tab->force_fields, nff, tab->ff_perm);
+            launch_overlapped(k_adj_p2g, (n + 127) / 128, 128, s, *prob, tab->instances, tab->materials, sp, adj,
+                              lame_bar, aw);
         }
     }
     return cuda_ok();
