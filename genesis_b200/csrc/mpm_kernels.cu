@@ -860,7 +860,9 @@ __device__ __forceinline__ void collide_rigid(const mpm_collider& c, const float
                                               float mass, const float* p, float* v, float* fout) {
     float sd, g[3], q[3], n[3];
     sdf_grad(c, sdf, eps, p, sd, g, q);
-    const float influence = fminf(expf(-sd / fmaxf(1e-10f, c.softness)), 1.f);
+    const float soft = fmaxf(1e-10f, c.softness);
+    if (sd > 2.4f * soft) return;  // influence < 0.1 (exp(-2.4) = 0.09): most nodes, without the exponential
+    const float influence = fminf(expf(-sd / soft), 1.f);
     if (!(influence > 0.1f)) return;
     unit_normal(c, eps, g, n);
     rigid_respond(c, eps, dt, mass, q, n, influence, v, fout);
@@ -923,7 +925,9 @@ __device__ __forceinline__ void collide_tool(const mpm_collider& c, const float*
         pv[i] = c.sdf_scale[i] * (c.rot[0 * 3 + i] * q[0] + c.rot[1 * 3 + i] * q[1] + c.rot[2 * 3 + i] * q[2]) + half;
     const float* vox = sdf_voxels + c.sdf_offset;
     const float sd = tool_sdf_at(vox, c.sdf_res, pv);
-    const float influence = fminf(expf(-sd / fmaxf(eps, c.softness)), 1.f);
+    const float soft = fmaxf(eps, c.softness);
+    if (sd > 2.4f * soft) return;  // influence < 0.1, as in collide_rigid
+    const float influence = fminf(expf(-sd / soft), 1.f);
     if (!(sd <= 0.f || influence > 0.1f)) return;
     // vel_collider (mesh.py:139-145): where the body point at p is one substep later, minus p,
     // over dt.  Written as ((E - I) q + dpos) / dt with (E - I) q = sin(th) k x q +
@@ -2092,13 +2096,10 @@ __global__ void k_nonfree_zero(mpm_problem prob, const mpm_instance* __restrict_
 
 // ---------------------------------------------------------------- grid op
 
-// constant-velocity kinematic motion of the colliders over one substep of their instance:
+// constant-velocity kinematic motion of a collider over one substep of its instance:
 // pos += lin_vel dt (a tool's origin then clamped to its floor, tool_entity.py:178-189),
 // rot = exp([ang_vel] dt) rot
-__global__ void k_advance_colliders(const mpm_instance* __restrict__ inst, int n_inst, mpm_collider* cs, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    mpm_collider& c = cs[i];
+__device__ __forceinline__ void advance_collider(const mpm_instance* inst, int n_inst, mpm_collider& c) {
     if (c.instance < 0 || c.instance >= n_inst) return;
     const float dt = inst[c.instance].dt;
 #pragma unroll
@@ -2271,10 +2272,11 @@ struct RecGrid {
 // node's momentum, mass and velocity (two kernels of their own before, a copy before and after)
 template <bool FF, bool REC = false>
 __global__ void __launch_bounds__(256, 4) k_grid_op(mpm_problem prob, const mpm_instance* __restrict__ inst, Ws w,
-                                                 const mpm_collider* __restrict__ colliders, int n_colliders,
+                                                 const mpm_collider* colliders, int n_colliders,
                                                  float* collider_force, const float* __restrict__ sdf_voxels,
                                                  const mpm_force_field* __restrict__ ffs, int n_ff,
-                                                 const int* __restrict__ ff_perm, int count_op, uint32_t* count, Grid old, RecGrid rec) {
+                                                 const int* __restrict__ ff_perm, int count_op, uint32_t* count, Grid old, RecGrid rec,
+                                                 mpm_collider* moving) {
     const int n_active = (int)*count;
     if (REC && blockIdx.x == 0 && threadIdx.x == 0) *rec.n_active = (uint32_t)n_active;
     const uint32_t ops = w.counters[CNT_GRID_OPS];
@@ -2352,14 +2354,22 @@ __global__ void __launch_bounds__(256, 4) k_grid_op(mpm_problem prob, const mpm_
     // the last CTA to finish resets the active-block count for the next p2g: every CTA read
     // the count into registers before this barrier, so no fence is needed; no CTA waits on
     // another
+    __shared__ bool last;
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (atomicAdd(&w.counters[CNT_DONE], 1u) == gridDim.x - 1) {
+        last = atomicAdd(&w.counters[CNT_DONE], 1u) == gridDim.x - 1;
+        if (last) {
             *count = 0u;
             if (old.mm) *old.n_active = 0u;
             w.counters[CNT_DONE] = 0u;
             if (count_op) w.counters[CNT_GRID_OPS] = ops + 1u;
         }
+    }
+    // and moves the colliders on (every CTA has used their poses): a kernel of its own before, 2 us a substep
+    if (moving) {
+        __syncthreads();
+        if (last)
+            for (int k = threadIdx.x; k < n_colliders; k += blockDim.x) advance_collider(inst, prob.n_instances, moving[k]);
     }
 }
 
@@ -2638,9 +2648,8 @@ static int launch_grid_op(const mpm_problem* prob, const mpm_tables* tab, void* 
                       : (rec ? k_grid_op<false, true> : k_grid_op<false, false>);
     k<<<ctas, 256, 0, s>>>(*prob, tab->instances, w, tab->colliders, nc, advance ? tab->collider_force : nullptr,
                            tab->sdf_voxels, nff > 0 ? tab->force_fields : nullptr, nff, nff > 0 ? tab->ff_perm : nullptr,
-                           advance ? 1 : 0, count, old ? *old : none, rec ? *rec : RecGrid{});
-    if (nc > 0 && advance)
-        k_advance_colliders<<<(nc + 63) / 64, 64, 0, s>>>(tab->instances, prob->n_instances, tab->colliders, nc);
+                           advance ? 1 : 0, count, old ? *old : none, rec ? *rec : RecGrid{},
+                           nc > 0 && advance ? tab->colliders : nullptr);
     return cuda_ok();
 }
 
