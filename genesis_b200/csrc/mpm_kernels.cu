@@ -1547,11 +1547,14 @@ __device__ __forceinline__ void scatter_flush(Tile& T, const Payload& o, const m
 #pragma unroll 1
                         for (int bz = lo[2]; bz <= hi[2]; ++bz) mark_block(w, inst, I, bx, by, bz, n_active);
             }
+            // nine nodes' independent arithmetic at a time: one node after another was 27 chains of
+            // some fifty dependent instructions
+            constexpr int kInner = CPIC ? 1 : 3;
 #pragma unroll 1
             for (int i = 0; i < 3; ++i)
-#pragma unroll 1
+#pragma unroll kInner
                 for (int j = 0; j < 3; ++j)
-#pragma unroll 1
+#pragma unroll kInner
                     for (int k = 0; k < 3; ++k) {
                         const int gx = o.base[0] + i, gy = o.base[1] + j, gz = o.base[2] + k;
                         if (gx < 0 || gy < 0 || gz < 0 || gx >= I.res[0] || gy >= I.res[1] || gz >= I.res[2]) {
