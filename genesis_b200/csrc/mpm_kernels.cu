@@ -2378,38 +2378,88 @@ __global__ void __launch_bounds__(256, 4) k_grid_op(mpm_problem prob, const mpm_
 
 // ---------------------------------------------------------------- state I/O
 
-__global__ void k_get_state(mpm_problem prob, mpm_particles par, float* pos, float* vel, float* C, float* F, float* Jp,
-                            uint8_t* active) {
+// Rows of W floats per particle (position, velocity, C, F) between registers, one particle per lane,
+// and an API-order array, through shared memory: consecutive lanes touch consecutive floats, so a
+// warp's access covers a few particles' 12- or 36-byte rows instead of 32 scattered words (W is odd,
+// so both views of the staging buffer are free of bank conflicts).  us against one word per lane (one
+// B200): whole state out 4M particles 241 against 543, 500k 29 / 64; in 159 / 182, 24 / 28.
+constexpr int IO_T = 256;  // threads of the state I/O kernels
+template <int W>
+__device__ __forceinline__ void rows_out(float* dst, const float* v, int g, int n, float* sm) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < W; ++c) sm[lane * W + c] = v[c];
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < W; ++t) {
+        const int f = t * 32 + lane, q = f / W;
+        const int gq = __shfl_sync(0xffffffffu, g, q);
+        if (q < n) dst[(int64_t)gq * W + (f - q * W)] = sm[f];
+    }
+}
+template <int W>
+__device__ __forceinline__ void rows_in(const float* src, float* v, int g, int n, float* sm) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < W; ++t) {
+        const int f = t * 32 + lane, q = f / W;
+        const int gq = __shfl_sync(0xffffffffu, g, q);
+        if (q < n) sm[f] = src[(int64_t)gq * W + (f - q * W)];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < W; ++c) v[c] = sm[lane * W + c];
+}
+
+__global__ void __launch_bounds__(IO_T) k_get_state(mpm_problem prob, mpm_particles par, float* pos, float* vel,
+                                                    float* C, float* F, float* Jp, uint8_t* active) {
+    __shared__ float stage[IO_T / 32][32 * 9];
+    float* sm = stage[threadIdx.x >> 5];
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= prob.n_particles) return;
-    const int g = par.gid[s];
+    const int n = min(32, prob.n_particles - (s & ~31));  // the warp's particles
+    if (n <= 0) return;
+    const bool in = s < prob.n_particles;
+    const int g = in ? par.gid[s] : 0;
     const int64_t st = par.state_stride;
-    for (int d = 0; d < 3; ++d) {
-        if (pos) pos[(int64_t)g * 3 + d] = par.state[(MPM_CH_X + d) * st + s];
-        if (vel) vel[(int64_t)g * 3 + d] = par.state[(MPM_CH_V + d) * st + s];
-    }
-    for (int k = 0; k < 9; ++k) {
-        if (C) C[(int64_t)g * 9 + k] = par.state[(MPM_CH_C + k) * st + s];
-        if (F) F[(int64_t)g * 9 + k] = par.state[(MPM_CH_F + k) * st + s];
-    }
+    float v[9];
+    auto load = [&](int ch, int w) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+            if (k < w) v[k] = in ? par.state[(ch + k) * st + s] : 0.f;
+    };
+    if (pos) load(MPM_CH_X, 3), rows_out<3>(pos, v, g, n, sm);
+    if (vel) load(MPM_CH_V, 3), rows_out<3>(vel, v, g, n, sm);
+    if (C) load(MPM_CH_C, 9), rows_out<9>(C, v, g, n, sm);
+    if (F) load(MPM_CH_F, 9), rows_out<9>(F, v, g, n, sm);
+    if (!in) return;
     if (Jp) Jp[g] = par.state[MPM_CH_JP * st + s];
     if (active) active[g] = (par.pflags[s] & MPM_PFLAG_ACTIVE) ? 1 : 0;
 }
 
-__global__ void k_set_state(mpm_problem prob, mpm_particles par, const float* pos, const float* vel, const float* C,
-                            const float* F, const float* Jp, const uint8_t* active) {
+__global__ void __launch_bounds__(IO_T) k_set_state(mpm_problem prob, mpm_particles par, const float* pos,
+                                                    const float* vel, const float* C, const float* F, const float* Jp,
+                                                    const uint8_t* active) {
+    __shared__ float stage[IO_T / 32][32 * 9];
+    float* sm = stage[threadIdx.x >> 5];
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= prob.n_particles) return;
-    const int g = par.gid[s];
+    const int n = min(32, prob.n_particles - (s & ~31));
+    if (n <= 0) return;
+    const bool in = s < prob.n_particles;
+    const int g = in ? par.gid[s] : 0;
     const int64_t st = par.state_stride;
-    for (int d = 0; d < 3; ++d) {
-        if (pos) par.state[(MPM_CH_X + d) * st + s] = pos[(int64_t)g * 3 + d];
-        if (vel) par.state[(MPM_CH_V + d) * st + s] = vel[(int64_t)g * 3 + d];
-    }
-    for (int k = 0; k < 9; ++k) {
-        if (C) par.state[(MPM_CH_C + k) * st + s] = C[(int64_t)g * 9 + k];
-        if (F) par.state[(MPM_CH_F + k) * st + s] = F[(int64_t)g * 9 + k];
-    }
+    float v[9];
+    auto store = [&](int ch, int w) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+            if (k < w && in) par.state[(ch + k) * st + s] = v[k];
+    };
+    if (pos) rows_in<3>(pos, v, g, n, sm), store(MPM_CH_X, 3);
+    if (vel) rows_in<3>(vel, v, g, n, sm), store(MPM_CH_V, 3);
+    if (C) rows_in<9>(C, v, g, n, sm), store(MPM_CH_C, 9);
+    if (F) rows_in<9>(F, v, g, n, sm), store(MPM_CH_F, 9);
+    if (!in) return;
     if (Jp) par.state[MPM_CH_JP * st + s] = Jp[g];
     if (active) par.pflags[s] = (uint8_t)((par.pflags[s] & ~MPM_PFLAG_ACTIVE) | (active[g] ? MPM_PFLAG_ACTIVE : 0));
 }
@@ -3613,7 +3663,7 @@ int mpm_get_state(const mpm_problem* prob, const mpm_particles* par, float* pos,
     if (rc) return rc;
     if ((rc = check_par(prob, par))) return rc;
     const int n = prob->n_particles;
-    if (n > 0) k_get_state<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(*prob, *par, pos, vel, C, F, Jp, active);
+    if (n > 0) k_get_state<<<(n + IO_T - 1) / IO_T, IO_T, 0, (cudaStream_t)stream>>>(*prob, *par, pos, vel, C, F, Jp, active);
     return cuda_ok();
 }
 
@@ -3623,7 +3673,7 @@ int mpm_set_state(const mpm_problem* prob, mpm_particles* par, const float* pos,
     if (rc) return rc;
     if ((rc = check_par(prob, par))) return rc;
     const int n = prob->n_particles;
-    if (n > 0) k_set_state<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(*prob, *par, pos, vel, C, F, Jp, active);
+    if (n > 0) k_set_state<<<(n + IO_T - 1) / IO_T, IO_T, 0, (cudaStream_t)stream>>>(*prob, *par, pos, vel, C, F, Jp, active);
     return cuda_ok();
 }
 
