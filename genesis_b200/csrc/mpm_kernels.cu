@@ -3863,8 +3863,13 @@ int mpm_graph_launch(void* graph, void* stream) {
 int mpm_graph_destroy(void* graph) {
     if (!graph) return MPM_E_INVALID;
     GraphHandle* h = (GraphHandle*)graph;
+    // A scene may be collected at any moment, also while this or another thread captures a stream; the
+    // release frees memory, which an unrelaxed capture would take for an error of its own
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     cudaGraphExecDestroy(h->exec);
     cudaGraphDestroy(h->graph);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     delete h;
     return MPM_OK;
 }

@@ -39,7 +39,7 @@ def _compare(a, b):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("runs,interval", [((1,), 50), ((2,), 50), ((3,), 50), ((4, 1, 2, 7), 50), ((60,), 25),
-                                           ((20, 13), 8), ((5, 5), 0)])
+                                           ((20, 13), 8), ((5, 5), 0), ((10,) * 12, 50), ((6, 6, 6, 6, 6), 8)])
 @pytest.mark.parametrize("graphs", [False, True])
 def test_runs_match_the_separate_kernels(runs, interval, graphs):
     rts = [_runtime([_desc(9), _desc(12, seed=6)], rot, sort_interval=interval, use_graphs=graphs)
@@ -101,3 +101,43 @@ def test_allocation_free_entry_takes_a_flagged_problem():
     b.sort_interval = 5
     b.substeps(7)
     _compare(a, b)
+
+
+@pytest.mark.gpu
+def test_graphs_are_released_while_another_stream_captures():
+    rt = _runtime([_desc(8)], True, sort_interval=20)
+    for _ in range(5):
+        rt.substeps(10)  # captured from the second time on
+    torch.cuda.synchronize()
+    assert rt._graphs
+    x = torch.zeros(4, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):  # (a scene collected inside somebody's capture)
+        x += 1
+        rt._drop_graphs()
+        x += 1
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x[0]) == 2.0 and not rt._graphs
+    rt.substeps(10)
+    assert rt.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_side", [8, 44])  # with the rotating grids, and enough particles for neither
+def test_short_runs_can_be_captured_by_the_caller(n_side):
+    rts = [R.runtime_from_descs([_desc(n_side)], sort_interval=50) for _ in range(2)]
+    for rt in rts:
+        for _ in range(5):
+            rt.substeps(10)  # phases 0, 10, .. 40
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            rts[0].substeps(10)
+        g.replay()
+    torch.cuda.current_stream().wait_stream(s)
+    rts[1].substeps(10)
+    torch.cuda.synchronize()
+    _compare(*rts)
