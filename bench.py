@@ -546,8 +546,8 @@ def run_ours(args, world, rank, local):
             "kernel_share": {k: round(v[0] * v[1] / prof_ms, 4) for k, v in kb.items()},
             "launches_per_substep": {k: round(v[2] / nsub, 4) for k, v in kb.items()},
             "timing": f"CUDA events between consecutive launch groups over {nsub} substeps of the same "
-                      "schedule (mpm_substeps_profile, no graph); kernel_ms is per launch group (a sort is 7 "
-                      "kernels)",
+                      "schedule (mpm_substeps_profile, no graph); kernel_ms is per launch group (a sort is 4 "
+                      "kernels, 7 above 40,000 blocks)",
             "profile_ms_per_substep": prof_ms / nsub,
             "substep_ms": step_sub_ms,
             "profile_vs_step": (prof_ms / nsub) / step_sub_ms,
