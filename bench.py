@@ -496,7 +496,11 @@ def run_ours(args, world, rank, local):
     kb, prof_ms = kernel_breakdown(rt, nsub)
     hbm, src = peaks()
     dom = max(kb, key=lambda k: kb[k][0] * kb[k][1])
-    bp, bc = BYTES[dom]
+    from genesis_b200 import _native as nat
+
+    # (the fused kernel is the whole substep where the runtime folds the grid op into it)
+    folded = dom == "g2p2g" and rt.prob.flags & nat.PROBF_ROTATE
+    bp, bc = SUBSTEP_BYTES if folded else BYTES[dom]
     alg = bp * d.n_particles + bc * n_act
     step_sub_ms = dev_ms / (args.steps * S)
     t_dom = kb[dom][0] * 1e-3

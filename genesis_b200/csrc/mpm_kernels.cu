@@ -3279,7 +3279,7 @@ static int substeps_impl(const mpm_problem* prob, const mpm_tables* tab, mpm_par
     }
     if ((rc = launch_p2g(prob, tab, par, ws, s))) return rc;
     mark(MPM_KIND_P2G);
-    const bool rotate = !pr && rotate_applies(prob, tab);
+    const bool rotate = rotate_applies(prob, tab);
     int32_t k = 0;  // substeps since the last p2g
     // the grid op that ends a stretch of substeps (before a re-sort, at the end)
     auto grid_op = [&]() {
@@ -3290,6 +3290,7 @@ static int substeps_impl(const mpm_problem* prob, const mpm_tables* tab, mpm_par
     for (int32_t i = 1; i < n; ++i) {
         if (!sort_due(i) && rotate) {
             if ((rc = launch_rotate(prob, tab, par, ws, ++k, s))) return rc;
+            mark(MPM_KIND_G2P2G);
             continue;
         }
         if ((rc = grid_op())) return rc;

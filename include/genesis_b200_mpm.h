@@ -448,13 +448,16 @@ int mpm_substeps_adjoint_recorded(const mpm_problem* prob, const mpm_tables* tab
  * (the stream is synchronised) ms_by_kind[k] holds the device milliseconds spent in kernels
  * of kind k and launches_by_kind[k] their number of kernel launches, both arrays of
  * MPM_N_KINDS entries.  Consecutive events bracket consecutive launches, so the kinds' times
- * add up to the run's device time.  The simulation advances exactly as with mpm_substeps.
+ * add up to the run's device time.  The simulation advances exactly as with mpm_substeps, by the
+ * same launches (an event between two kernels keeps them from overlapping).
  * No counterpart in the reference (its Taichi kernels are timed by its own profiler). */
 #define MPM_KIND_SORT 0        /* the kernels of mpm_sort_particles (4; 7 above 40,000 blocks) */
 #define MPM_KIND_P2G 1
 #define MPM_KIND_GRID_OP 2
 #define MPM_KIND_G2P 3
-#define MPM_KIND_G2P2G 4       /* g2p of one substep fused with p2g of the next */
+#define MPM_KIND_G2P2G 4       /* g2p of one substep fused with p2g of the next (and the grid op between
+                                  them, where MPM_PROBF_ROTATE applies: MPM_KIND_GRID_OP is then one
+                                  launch a run) */
 #define MPM_N_KINDS 5
 int mpm_substeps_profile(const mpm_problem* prob, const mpm_tables* tab, mpm_particles* par, void* workspace,
                          int32_t n_substeps, int32_t sort_interval, int64_t first_substep, float* ms_by_kind,

@@ -141,3 +141,18 @@ def test_short_runs_can_be_captured_by_the_caller(n_side):
     rts[1].substeps(10)
     torch.cuda.synchronize()
     _compare(*rts)
+
+
+@pytest.mark.gpu
+def test_profile_times_the_schedule_that_runs():
+    for rot in (True, False):
+        a, b = (_runtime([_desc(9)], rot, sort_interval=8) for _ in range(2))
+        prof = {k: n for k, (ms, n) in a.profile_substeps(20).items()}
+        b.substeps(20)
+        _compare(a, b)
+        # 8 + 8 + 4 substeps, each run from its sort; the grid op by itself only at a run's end
+        # where it is folded into the fused kernel
+        assert prof == {"sort": 3 * 4, "p2g": 3, "g2p": 3, "g2p2g": 7 + 7 + 3, "grid_op": 3 if rot else 20}
+        a.substeps(12)  # and the grids are left clean
+        b.substeps(12)
+        _compare(a, b)
