@@ -25,6 +25,11 @@ ROTATE_MAX_PARTICLES = 300_000
 ROTATE_MAX_BYTES = 1 << 30  # of extra grids (32 bytes per node)
 
 
+def rotate_bytes(n_blocks: int) -> int:
+    """Bytes of the two extra grids: momentum and mass of every node."""
+    return 2 * 16 * nat.MPM_BLOCK ** 3 * n_blocks
+
+
 @dataclass
 class InstanceSpec:
     """Constants of one scene (MPMSolver.__init__, mpm_solver.py:31-78)."""
@@ -258,12 +263,7 @@ class MPMRuntime:
             cpic_normal=self.cpic_normal.data_ptr() if self.cpic_normal is not None else None,
             cpic_sep=self.cpic_sep.data_ptr() if self.cpic_sep is not None else None,
         )
-        # (a differentiated plastic rollout keeps the separate kernels: its gradient jumps where a return
-        # mapping switches branch, which another order of the grid's sums can cause)
-        plastic = any(m.kind in (nat.MAT_ELASTOPLASTIC, nat.MAT_SAND, nat.MAT_SNOW) for m in mats)
-        if (P == 128 and self.n <= ROTATE_MAX_PARTICLES and not colliders and not force_fields
-                and not (per_particle_lame and plastic) and 32 * 64 * self.n_blocks <= ROTATE_MAX_BYTES):
-            self.prob.flags |= nat.PROBF_ROTATE
+        self._set_rotate()
         nbytes = C.c_uint64()
         nat.check("mpm_workspace_bytes", self.lib.mpm_workspace_bytes(C.byref(self.prob), C.byref(nbytes)))
         self.workspace_bytes = int(nbytes.value)
@@ -272,6 +272,22 @@ class MPMRuntime:
         self._call("mpm_workspace_init", C.byref(self.prob), self._ws, _cuda_stream_handle())
 
     # ------------------------------------------------------------------ utils
+    def rotate_eligible(self) -> bool:
+        """Whether runs of substeps of this problem, at 128 particles per work item, fold the grid op
+        into the particle kernel: few enough particles, nothing but gravity and the boundary on the
+        grid.  (A differentiated plastic rollout keeps the separate kernels, the ones that its reverse
+        pass records: a return mapping's branch can depend on the order of the grid's sums.)"""
+        plastic = any(m.kind in (nat.MAT_ELASTOPLASTIC, nat.MAT_SAND, nat.MAT_SNOW) for m in self._mats)
+        return (self.n <= ROTATE_MAX_PARTICLES and not self.n_colliders and not self.n_force_fields
+                and not (self.mu_p is not None and plastic) and rotate_bytes(self.n_blocks) <= ROTATE_MAX_BYTES)
+
+    def _set_rotate(self):
+        """The problem's MPM_PROBF_ROTATE for its particles per work item."""
+        if self.prob.chunk_particles == 128 and self.rotate_eligible():
+            self.prob.flags |= nat.PROBF_ROTATE
+        else:
+            self.prob.flags &= ~nat.PROBF_ROTATE
+
     def _call(self, name, *args):
         rc = getattr(self.lib, name)(*args)
         nat.check(name, rc)
@@ -549,9 +565,12 @@ class MPMRuntime:
             nat.check("mpm_max_chunks", self.lib.mpm_max_chunks(self.n, self.n_blocks, P, C.byref(mc)))
             self.prob.chunk_particles = P
             self.prob.max_chunks = mc.value
+            flags = self.prob.flags
+            self._set_rotate()
             nbytes = C.c_uint64()
             nat.check("mpm_workspace_bytes", self.lib.mpm_workspace_bytes(C.byref(self.prob), C.byref(nbytes)))
-            if int(nbytes.value) > self.workspace.numel():
+            # (a smaller one too where the extra grids came off: they are half of the grid memory)
+            if int(nbytes.value) > self.workspace.numel() or flags & ~self.prob.flags & nat.PROBF_ROTATE:
                 self.workspace = torch.empty(int(nbytes.value), dtype=torch.uint8, device=self.device)
                 self._ws = C.c_void_p(self.workspace.data_ptr())
             self.workspace_bytes = int(nbytes.value)

@@ -156,3 +156,24 @@ def test_profile_times_the_schedule_that_runs():
         a.substeps(12)  # and the grids are left clean
         b.substeps(12)
         _compare(a, b)
+
+
+@pytest.mark.gpu
+def test_retune_takes_the_folded_kernel_on_and_off(monkeypatch):
+    a = R.runtime_from_descs([_desc(9), _desc(12, seed=6)], sort_interval=16, chunk_particles=256)
+    b = _runtime([_desc(9), _desc(12, seed=6)], False, sort_interval=16)
+    assert not a.prob.flags & nat.PROBF_ROTATE
+    plain = a.workspace_bytes
+    for P, rot in ((256, False), (128, True), (256, False), (128, True)):
+        a.retune(chunk_particles=P)
+        assert bool(a.prob.flags & nat.PROBF_ROTATE) == rot
+        assert a.workspace.numel() >= a.workspace_bytes
+        assert rot or a.workspace.numel() == plain  # the extra grids are given back
+        for rt in (a, b):
+            rt.substeps(11)
+            rt.substeps(6)
+        _compare(a, b)
+    monkeypatch.setattr(R, "ROTATE_MAX_PARTICLES", 2000)  # 2,457 particles: too many
+    a.retune(chunk_particles=256)
+    a.retune(chunk_particles=128)
+    assert not a.prob.flags & nat.PROBF_ROTATE
