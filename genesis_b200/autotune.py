@@ -7,8 +7,8 @@ interval and the persistent CTA count (grid_ctas; the candidates are given per S
 leaves slots free for a concurrent stream, 14 per SM is two waves of the 128-particle
 kernels, which evens out the tail when the work items are few and uneven).  The grid block edge is fixed at 4 nodes (it sets
 the block-major grid layout and the 8^3 shared tile).  Results are cached per problem
-signature (particle and grid-block counts rounded to powers of two) in a JSON file so a
-served or batched workload tunes once.
+signature (particle and grid-block counts rounded to powers of two, whether the problem may fold
+the grid op into the particle kernel) in a JSON file so a served or batched workload tunes once.
 """
 
 from __future__ import annotations
@@ -29,9 +29,16 @@ DEFAULT_CANDIDATES = {
 _lock = threading.Lock()
 
 
+# Part of the key: raised when the substep schedule changes what the candidates cost, so that choices
+# timed on another schedule are not applied (2: the grid op folded into the particle kernel).
+SCHEDULE = 2
+
+
 def signature(rt) -> str:
     b = lambda x: 1 << max(0, int(math.ceil(math.log2(max(1, x)))))
-    return f"n{b(rt.n)}_blk{b(rt.n_blocks)}_inst{b(len(rt.specs))}"
+    # whether the 128-particle candidates fold the grid op: not settled by the rounded sizes
+    # (262,145 to 524,288 particles share one, the limit is 300,000), colliders, force fields or Lame parameters
+    return f"s{SCHEDULE}_n{b(rt.n)}_blk{b(rt.n_blocks)}_inst{b(len(rt.specs))}_rot{int(rt.rotate_eligible())}"
 
 
 def _cache_path():
