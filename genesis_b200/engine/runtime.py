@@ -97,6 +97,8 @@ class MPMRuntime:
     chunk_particles : particles per p2g/g2p work item (128, 256 or 512)
     sort_interval : re-bin particles every this many substeps
     per_particle_lame : allocate per-particle (mu, lam) overrides
+    rotate : allow the two extra grids (rotate_bytes) of problems that fold the grid op into the
+        particle kernel
     """
 
     def __init__(
@@ -113,6 +115,7 @@ class MPMRuntime:
         cpic: bool = False,
         force_fields: list | None = None,
         ff_perm: np.ndarray | None = None,
+        rotate: bool = True,
     ):
         if not torch.cuda.is_available():
             raise RuntimeError("genesis_b200 needs a CUDA device (sm_100a); there is no CPU path")
@@ -121,6 +124,7 @@ class MPMRuntime:
         self.specs = list(specs)
         self.sort_interval = int(sort_interval)
         self.use_graphs = bool(use_graphs)
+        self.rotate = bool(rotate)
         self._graphs: dict = {}
         self._runs_seen: set = set()  # runs shorter than the sort interval that came once
         self._run_graph_substeps = 0
@@ -278,7 +282,7 @@ class MPMRuntime:
         grid.  (A differentiated plastic rollout keeps the separate kernels, the ones that its reverse
         pass records: a return mapping's branch can depend on the order of the grid's sums.)"""
         plastic = any(m.kind in (nat.MAT_ELASTOPLASTIC, nat.MAT_SAND, nat.MAT_SNOW) for m in self._mats)
-        return (self.n <= ROTATE_MAX_PARTICLES and not self.n_colliders and not self.n_force_fields
+        return (self.rotate and self.n <= ROTATE_MAX_PARTICLES and not self.n_colliders and not self.n_force_fields
                 and not (self.mu_p is not None and plastic) and rotate_bytes(self.n_blocks) <= ROTATE_MAX_BYTES)
 
     def _set_rotate(self):

@@ -23,7 +23,7 @@ import torch
 
 from . import _native as nat
 from . import workloads as W
-from .engine.runtime import MPMRuntime, spec_from_desc
+from .engine.runtime import MPMRuntime, rotate_bytes, spec_from_desc
 from .materials import MPM
 
 
@@ -200,8 +200,11 @@ class MPMServer:
             for k in parts:
                 v = slot.state[k]
                 parts[k].append(v.reshape(v.shape[0], -1) if k in ("C", "F") else v)
+        # (128-particle layouts may take two more grids, which the requests' estimates do not hold:
+        # where the budget has no room for them the layout does without)
+        extra = rotate_bytes(sum(sp.n_blocks for sp in specs))
         self.rt = MPMRuntime(specs, chunk_particles=self.chunk, sort_interval=self.sort_interval,
-                             use_graphs=self.use_graphs)
+                             use_graphs=self.use_graphs, rotate=self.queue.in_use + extra <= self.queue.budget)
         self.rt.load_state(torch.cat(parts["pos"]), torch.cat(parts["vel"]), torch.cat(parts["C"]),
                            torch.cat(parts["F"]), torch.cat(parts["Jp"]), torch.cat(parts["active"]),
                            torch.cat(parts["mat"]))

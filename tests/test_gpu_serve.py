@@ -78,3 +78,25 @@ def test_batched_admission_keeps_results():
         assert r.error is None, r.error
         pos, _ = _alone(q.scene)
         assert np.abs(r.pos - pos).max() <= 1e-5, r.rid
+
+
+def test_extra_grids_stay_within_the_budget():
+    """128-particle layouts of small requests take two more grids where the budget has room for them,
+    and do without where it has not: the request is served either way."""
+    from genesis_b200 import _native as nat
+
+    d = W.elastic_cube(n_side=12, n_substeps=20)
+    need = serve.estimate_bytes(d, 128)
+    results = []
+    for budget, rot in ((1.05 * need, False), (3.0 * need, True)):
+        srv = serve.MPMServer(budget_bytes=budget, tick_substeps=10, chunk_particles=128)
+        assert srv.queue.push(W.Request(0, 0.0, d)) is None
+        (req, n), = srv.queue.pop_admissible(0)
+        srv._repack([serve._Slot(req, d.n_substeps, n)])
+        assert bool(srv.rt.prob.flags & nat.PROBF_ROTATE) == rot
+        assert srv.rt.memory_bytes() <= budget
+        srv = serve.MPMServer(budget_bytes=budget, tick_substeps=10, chunk_particles=128)
+        (r,) = srv.serve([W.Request(0, 0.0, d)], realtime=False)
+        assert r.error is None
+        results.append(r.pos)
+    assert np.abs(results[0] - results[1]).max() <= 1e-6
