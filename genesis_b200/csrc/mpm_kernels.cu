@@ -1980,9 +1980,8 @@ __global__ void __launch_bounds__(P, kP2GCtasPerSM<P>) k_g2p2g(P2GArgs a) {
 // kernel before.  us per substep against g2p2g + grid op (49 substeps, one B200): 1k elastic
 // particles 8.0 against 14.5, 32k 10.1 / 16.0, 16 environments of 2k muscle particles 11.4 / 17.5,
 // 80k snow 17.3 / 23.3, 125k sand 23.9 / 28.8, 216k elastic 31.3 / 36.7, 288k 41.1 / 43.9.
-constexpr int kRotateClearers = 148;
 template <int P, bool MUSCLE>
-__global__ void __launch_bounds__(P, kP2GCtasPerSM<P>) k_g2p2g_rotate(P2GArgs a, Grid old, uint32_t* n_out) {
+__global__ void __launch_bounds__(P, kP2GCtasPerSM<P>) k_g2p2g_rotate(P2GArgs a, Grid old, uint32_t* n_out, int n_sms) {
     __shared__ VelTile VT;
     __shared__ Tile T;
     __shared__ Stash<P> SH;
@@ -1991,7 +1990,7 @@ __global__ void __launch_bounds__(P, kP2GCtasPerSM<P>) k_g2p2g_rotate(P2GArgs a,
     // CTAs beyond the work items (and beyond one per SM, to clear the old grid) leave at once: left
     // waiting they would hold the places of the next kernel's CTAs, which then pile up on a few SMs
     // (32k particles: 14.0 us per substep with them, 9.9 without)
-    const int workers = min((int)gridDim.x, max(n_chunks, kRotateClearers));
+    const int workers = min((int)gridDim.x, max(n_chunks, n_sms));
     if ((int)blockIdx.x >= workers) return;
     const int64_t st = a.par.state_stride;
     float* __restrict__ S = a.par.state;
@@ -2749,7 +2748,7 @@ static int launch_rotate(const mpm_problem* prob, const mpm_tables* tab, mpm_par
     a.w.active = out.active;
     const int ctas = persistent_ctas(prob, d->occ_g2p2g[0]);
     launch_overlapped(par->actu ? k_g2p2g_rotate<128, true> : k_g2p2g_rotate<128, false>, ctas, 128, s, a, old,
-                      out.n_active);
+                      out.n_active, d->sms);
     return cuda_ok();
 }
 
