@@ -1144,9 +1144,7 @@ __device__ __forceinline__ void particle_update(const mpm_instance& I, const mpm
         Jpn = Jp;
     } else {
         float U[9], Sg[3], V[9];
-        // differentiable rollouts (per-particle Lame parameters) keep the order that the adjoint's
-        // SVD takes, so both see the same rounding: plastic flow amplifies it along the rollout
-        svd3(Ft, U, Sg, V, needs_uv(m, mu), par.mu_p != nullptr);
+        svd3(Ft, U, Sg, V, needs_uv(m, mu));
         J = Sg[0] * (Sg[1] * Sg[2]);
         constitutive(m, mu, lam, I.eps, J, Ft, U, Sg, V, Jp, Fn, Jpn, stress);
     }

@@ -116,3 +116,42 @@ def test_svd_reconstruction_on_ill_conditioned_F():
         # s_0 over s_i (forming B = A V in float32 already costs that), whichever is larger
         bound = np.where(low[sel], np.maximum(1e-5, 2.0**-22 * s0 / s[sel]), 0.0).sum(1)
         assert (jrel <= np.maximum(bound, 1e-6)).all(), (name, jrel.max(), bound.max())
+
+
+def _stretched(rng, sig):
+    n = len(sig)
+    F = _rot(rng, n) @ (sig[:, :, None] * np.swapaxes(_rot(rng, n), 1, 2))
+    return F.astype(np.float32).astype(np.float64)
+
+
+@pytest.mark.parametrize("ratio", [1.4, 2.0, 3.9])
+def test_moderate_stretches_lose_nothing_off_the_diagonal(ratio):
+    """U S V^T of stretches of up to 4 : 1 in the float64 basis: the entries off the diagonal are the
+    large columns' remainders in the small ones' directions, a rounding (6e-8) or so of s_0 where the
+    large columns are orthogonalised first, the ratio times that where a small one is.  Root mean
+    square over 3,375 particles within 1e-7."""
+    rng = np.random.default_rng(3)
+    n = 3375
+    t = rng.uniform(0.0, 1.0, size=(n, 3))
+    t[:, 0], t[:, 1] = 0.0, 1.0
+    sig = np.take_along_axis(1.1 * ratio ** (t - 0.5), np.argsort(rng.random((n, 3)), 1), 1)
+    F = _stretched(rng, sig)
+    U, s, Vt = np.linalg.svd(F)
+    E = np.swapaxes(U, 1, 2) @ (_run(F) - F) @ np.swapaxes(Vt, 1, 2)
+    E[:, [0, 1, 2], [0, 1, 2]] = 0.0
+    rms = np.sqrt((E ** 2).mean())
+    print(f"\n[svd] ratio {ratio}: rms off the diagonal {rms:.2e}")
+    assert rms <= 1e-7
+
+
+@pytest.mark.parametrize("sig", [(1.0, 1.0, 1e-2), (1.3, 0.9, 0.2), (2.8, 1.0, 1.0)])
+def test_liquid_volume_of_stretched_particles(sig):
+    """An inviscid Liquid takes J = det F_tmp alone, with no rotation to separate the columns, and writes
+    F_new = J^(1/3) I.  Its relative error: a rounding (6e-8) of s_0 in the smallest singular value and
+    a few in the others; three times 6e-8 s_0 / s_2 + 1e-6 is allowed."""
+    rng = np.random.default_rng(8)
+    F = _stretched(rng, np.tile(np.array(sig), (3375, 1)))
+    Fn = _run(F, ("liquid", dict(E=1e5, nu=0.2)))
+    err = np.abs(Fn[:, 0, 0] ** 3 / np.linalg.det(F) - 1.0).max()
+    print(f"\n[svd] liquid {sig}: J rel. err {err:.2e}")
+    assert err <= 3 * 6e-8 * max(sig) / min(sig) + 1e-6
