@@ -2839,7 +2839,8 @@ __device__ __forceinline__ void tri_solid_angle(const float* p, const float* a, 
     const float ra[3] = {a[0] - p[0], a[1] - p[1], a[2] - p[2]};
     const float rb[3] = {b[0] - p[0], b[1] - p[1], b[2] - p[2]};
     const float rc[3] = {c[0] - p[0], c[1] - p[1], c[2] - p[2]};
-    // 1 ulp square roots: only which side of 1/2 the sum of angles lies on is used
+    // approximate square roots (rsqrt.approx, 2^-22.9 relative, and a rounding): only which side of 1/2
+    // the sum of angles lies on is used
     auto root = [](float x) { return x * rsqrt_ftz(fmaxf(x, 1e-37f)); };
     const float la = root(ra[0] * ra[0] + ra[1] * ra[1] + ra[2] * ra[2]);
     const float lb = root(rb[0] * rb[0] + rb[1] * rb[1] + rb[2] * rb[2]);
@@ -2896,13 +2897,13 @@ struct Winding {
 //      than kSdfNear h is summed per node and the others' taken at q, with their bound.
 //   3. Where that leaves a node's side open (a winding number near 1/2: open meshes), every face is
 //      summed per node.
-// us against the loop over all pairs, one node per thread (one B200): 96^3 nodes x 1,280 faces 850
-// against 7,315; 128^3 x 2,300 2,740 against 29,700; 64^3 x 1,280 514 against 2,325.
+// us against the loop over all pairs, one node per thread (one B200): 96^3 nodes x 1,280 faces 625
+// against 7,323; 128^3 x 2,300 2,032 against 29,692; 64^3 x 1,280 410 against 2,335.
 constexpr int SDF_T = 256;
-// faces nearer than this many h are summed per node (96^3 nodes, 1,280 faces: 6 850 us, 4 1,218 us,
-// 3 1,987 us: below 6 the bound leaves more bricks to step 3)
+// faces nearer than this many h are summed per node (96^3 nodes, 1,280 faces: 6 625 us, 4 875 us,
+// 3 1,451 us: below 6 the bound leaves more bricks to step 3)
 constexpr float kSdfNear = 6.f;
-constexpr int64_t kSdfBrickNodes = 75000;  // about 42^3; the two kernels meet between 40^3 and 48^3
+constexpr int64_t kSdfBrickNodes = 75000;  // about 42^3 (1,280 faces: nodes 598 us, bricks 694; 48^3: 883, 516)
 constexpr int SDF_REC = 17;  // a, b, c, n, bounding sphere centre and radius, area
 
 struct SdfGrid {
@@ -2955,8 +2956,8 @@ __device__ __forceinline__ void sdf_stage(const float* __restrict__ V, int nv, c
 // Grids too small to fill the GPU with bricks (kSdfBrickNodes): one warp per node, its lanes
 // splitting the faces.  The winding number is the lanes' sum; the distance skips faces whose bounding
 // sphere lies beyond the nearest distance so far.  A brick of a coarse grid is also large against
-// the mesh, so that its bounds settle little.  us against bricks: 32^3 nodes x 1,280 faces 270 against 607, 24^3 x
-// 1,140 114 against 611; 48^3 x 1,280 898 against 611.
+// the mesh, so that its bounds settle little.  us against bricks: 32^3 nodes x 1,280 faces 280 against 532, 24^3 x
+// 1,140 124 against 536; 48^3 x 1,280 883 against 516.
 __global__ void __launch_bounds__(SDF_T) k_sdf_nodes(const float* __restrict__ V, int nv, const int* __restrict__ Fc,
                                                      int nf, SdfGrid G, float* __restrict__ out) {
     __shared__ float rec[SDF_REC][SDF_T];

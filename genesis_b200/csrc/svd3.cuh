@@ -33,9 +33,12 @@ constexpr int kSvdUnroll = GBM_SVD_UNROLL;
 #define GBM_SVD_TOL 1e-7f
 #endif
 
-// Approximate reciprocal square root and quotient, flushing subnormals: the arguments below are
-// kept above 1e-37 (or the result is selected away), and the default forms spend three to four
-// instructions each on scaling subnormal inputs.
+// Approximate reciprocal square root and quotient, flushing subnormals, for arguments that are no
+// subnormals (or whose result is selected away): the default forms spend three to four instructions
+// each on scaling them.  The roots' arguments are kept above 1e-37.  A rotation's divisor is at least
+// 2e-18 in jacobi_pq (|apq| > 1e-18); in onesided_pq |apq| > 1e-30 bounds the longer column's squared
+// length, of which the difference d is 0 or an ulp (5e-38) and more, and r2 adds 0 or 4e-27 and more.
+// (A divisor of 0, two such columns of one length below 1e-11, gives NaN in either form.)
 __device__ __forceinline__ float rsqrt_ftz(float x) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -153,7 +156,7 @@ __device__ __forceinline__ void cofactor3(const float* A, float* K) {
 // sixty instructions at the strains of a running scene, where the SVD takes about seven hundred.
 // The whole warp goes one way: returns false (nothing usable) where a lane has det A <= 0, is too
 // ill-conditioned for the determinant in float32 (|A|_F^6 >= 108 det^2: singular values (a, 1, 1)
-// pass for a in [0.3, 2.8]), or has not converged.
+// pass for a in [0.29, 2.68]), or has not converged.
 __device__ __forceinline__ bool polar3(const float* A, bool want_R, float* R, float& J) {
     const unsigned lanes = __activemask();
     float K[9];
