@@ -128,6 +128,7 @@ class MPMRuntime:
         self._graphs: dict = {}
         self._runs_seen: set = set()  # runs shorter than the sort interval that came once
         self._run_graph_substeps = 0
+        self._run_credit = 1.0  # captures of such runs that the runs so far pay for
         self._count = 0  # substeps executed
         self._nonfree = False
         self._dirty = False  # positions written since the last sort
@@ -667,12 +668,20 @@ class MPMRuntime:
 
     def _run_graph(self, m: int, K: int, phase: int):
         """A graph of the m substeps from `phase` of the sort interval, captured when such a run comes
-        for the second time (a scene stepped a few substeps at a time repeats its runs); None before
-        that, once the graphs hold RUN_GRAPH_SUBSTEPS, and inside a caller's own stream capture.  Launch by launch a substep's boundaries
-        cost more: 500k particles 89.7 us per substep against 83.8, 56k sand with a collider 28.2
-        against 21.0."""
+        again (a scene stepped a few substeps at a time repeats its runs) and the short runs so far
+        pay for the capture; None before that, once the graphs hold RUN_GRAPH_SUBSTEPS, and inside a
+        caller's own stream capture.
+
+        A capture takes 130-370 us and pays after 10-18 replays where the grid op is folded into the
+        particle kernel, whose launches overlap anyway (12 us a run), and after 30-110 substeps where
+        it is not (4-6 us a substep: 500k particles 89.7 us launch by launch against 83.8, 56k sand with
+        a collider 28.2 against 21.0).  So every 16 runs, or 128 substeps, pay for one graph, the first
+        being free: step sizes that meet the sort interval at dozens of phases would otherwise capture
+        dozens of graphs before the first is replayed (22k sand, 200 steps of 7 substeps: 38.7 ms with
+        a graph for every run that came twice, 30.8 without graphs)."""
         if torch.cuda.is_current_stream_capturing():
             return None  # the caller captures the launches themselves
+        self._run_credit += 1 / 16 if self.prob.flags & nat.PROBF_ROTATE else m / 128
         key = ("run", m, phase, K, self.prob.flags)
         g = self._graphs.get(key)
         if g is None:
@@ -680,11 +689,12 @@ class MPMRuntime:
                 if len(self._runs_seen) < 4 * K:
                     self._runs_seen.add(key)
                 return None
-            if self._run_graph_substeps + m > self.RUN_GRAPH_SUBSTEPS:
+            if self._run_credit < 1 or self._run_graph_substeps + m > self.RUN_GRAPH_SUBSTEPS:
                 return None
             g = self._capture(m, K, phase)
             self._graphs[key] = g
             self._run_graph_substeps += m
+            self._run_credit -= 1
         return g
 
     def _capture(self, n: int, K: int, first: int):

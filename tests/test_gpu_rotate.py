@@ -177,3 +177,26 @@ def test_retune_takes_the_folded_kernel_on_and_off(monkeypatch):
     a.retune(chunk_particles=256)
     a.retune(chunk_particles=128)
     assert not a.prob.flags & nat.PROBF_ROTATE
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rotate", [True, False])
+def test_short_runs_pay_for_their_graphs(rotate):
+    """200 runs of 7 substeps meet a sort interval of 50 at dozens of phases; a loop of 10 meets it at five."""
+    a, b = _runtime([_desc(8)], rotate, sort_interval=50), _runtime([_desc(8)], rotate, sort_interval=50)
+    b.use_graphs = False
+    runs = 0
+    for _ in range(200):
+        runs += 1 if a._count % 50 + 7 <= 50 else 2
+        for rt in (a, b):
+            rt.substeps(7)
+        if rotate:
+            assert len(a._graphs) <= 1 + runs / 16
+        else:
+            assert len(a._graphs) <= 1 + a._count / 128
+    assert len(a._graphs) >= 5
+    _compare(a, b)
+    c = _runtime([_desc(8)], rotate, sort_interval=50)
+    for _ in range(120):
+        c.substeps(10)
+    assert len(c._graphs) == 5
